@@ -34,6 +34,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 OUT = os.path.join(HERE, "_ref")
 # the reference checkout: VXR_REFERENCE, else where this container mounts it
 DEFAULT_REF = os.environ.get("VXR_REFERENCE", "/root/reference")
+if not os.path.isfile(os.path.join(DEFAULT_REF, "template", "common.h")):
+    # an empty mount point is no checkout: name a folder that does not exist in it, so
+    # every "is the reference there" test says no
+    DEFAULT_REF = os.path.join(DEFAULT_REF, "template")
 
 # tools.cl functions on the render path (the rest of tools.cl is TAA / tonemapping /
 # editor code that the path never reaches)
