@@ -499,9 +499,11 @@ typedef struct vxr_tuning {
     uint32_t tile_x, tile_y;       /* threads of a pixel-stage block; tile_x * tile_y a multiple of 32, <= 256 */
     uint32_t persistent;           /* pixel stages: 1 = resident blocks pull tiles from a queue, 0 = one block per tile */
     uint32_t shadow_refill;        /* shadow tracer: idle lanes of a warp (1..32) that trigger a refill from the queue */
-    uint32_t shadow_burst;         /* shadow tracer: cell visits per lane between refill checks (1..64) */
+    uint32_t shadow_burst;         /* shadow tracer: grid-cell visits per lane between refill checks (1..64, in steps of 4) */
     uint32_t list_blocks_per_sm;   /* hit-list kernels (candidates, temporal, shading requests): blocks per SM (1..64) */
-    uint32_t occupancy;            /* 1: shadow tracer and candidate kernels capped in registers for more warps per SM */
+    uint32_t occupancy;            /* 1: candidate kernel capped in registers for more warps per SM */
+    /* the next three belong to the tracer that walks a ray's cells of all levels in one
+       lane; any of them set selects it (the default tracer walks bricks by whole warps) */
     uint32_t shadow_schedule;      /* shadow tracer: 0 every lane steps each round, 1 only the lanes at the DDA level most lanes are at */
     uint32_t shadow_early_out;     /* shadow tracer: 1 stops a walk, as occluded, once its step budget cannot reach the emitter */
     uint32_t brick_cache;          /* shadow tracer: bricks whose opacity masks each CTA keeps in shared memory (0 off, 128..2048 a power of two) */

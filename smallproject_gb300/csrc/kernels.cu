@@ -25,8 +25,9 @@
 // light models): pixel stages are persistent blocks pulling screen tiles from a work queue;
 // the candidate loop, the temporal step and the shading request run over a compacted
 // list of hit pixels; and every shadow ray goes through one persistent tracer whose
-// lanes take a new ray as soon as theirs ends. Each pixel's arithmetic is unchanged,
-// so results are the same bit for bit whatever order pixels and rays are processed in.
+// lanes take a new ray as soon as theirs ends and whose warps walk bricks together. Each
+// pixel's arithmetic is unchanged, so results are the same bit for bit whatever order
+// pixels and rays are processed in.
 #include <algorithm>
 #include <cstdint>
 #include <map>
@@ -73,8 +74,8 @@ __global__ void build_uber_kernel(const uint32_t* __restrict__ grid, uint8_t* ub
 }
 
 // Per brick the boxes of its opaque voxels (type nibble 15) and of its non-zero voxels,
-// packed as World::bbox describes: one warp per brick, 16 voxels a lane, min / max
-// reductions over the warp.
+// packed as World::bbox describes, and its opacity mask (World::bmask): one warp per brick,
+// 16 voxels a lane, min / max reductions over the warp, a ballot per mask word.
 __device__ __forceinline__ uint32_t warp_box(bool any, const uint32_t lo[3], const uint32_t hi[3]) {
     const bool anyw = __any_sync(0xffffffffu, any);
     uint32_t box = 0u;
@@ -86,7 +87,8 @@ __device__ __forceinline__ uint32_t warp_box(bool any, const uint32_t lo[3], con
 }
 // (list: the bricks to do, or null for bricks 0 .. n - 1)
 __global__ void build_brick_boxes_kernel(const uint32_t* __restrict__ bricks, const uint32_t* __restrict__ list,
-                                         uint32_t n, uint32_t* __restrict__ bbox, uint32_t* __restrict__ bbox0) {
+                                         uint32_t n, uint32_t* __restrict__ bbox, uint32_t* __restrict__ bbox0,
+                                         uint32_t* __restrict__ bmask) {
     const size_t item = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (item >= n) return;   // whole warps leave together (blockDim a multiple of 32)
     const size_t brick = list ? (size_t)__ldg(list + item) : item;
@@ -97,7 +99,10 @@ __global__ void build_brick_boxes_kernel(const uint32_t* __restrict__ bricks, co
         const uint32_t e = i * 32u + lane;   // coalesced: a warp reads 32 consecutive voxels
         const uint32_t v = __ldg(bricks + brick * 512u + e);
         const uint32_t c[3] = {e & 7u, (e >> 3) & 7u, e >> 6};
-        if (((v & 0xf000u) >> 12) == 15u) {
+        const bool opaque = ((v & 0xf000u) >> 12) == 15u;
+        const uint32_t word = __ballot_sync(0xffffffffu, opaque);
+        if (lane == i) bmask[brick * 16u + i] = word;
+        if (opaque) {
             for (int a = 0; a < 3; a++) { lo[a] = min(lo[a], c[a]); hi[a] = max(hi[a], c[a]); }
             any = true;
         }
@@ -122,21 +127,27 @@ __global__ void commit_bricks_kernel(const uint32_t* __restrict__ list, const ui
     reinterpret_cast<uint4*>(bricks + (size_t)b * 512u)[threadIdx.x] = v;
 }
 
-// Per uber cell the box of its non-zero voxels (World::ubox0): brick-less non-zero grid
-// cells count whole, bricks with their non-zero box (bbox0, built before).
-__global__ void build_uber_boxes_kernel(const uint32_t* __restrict__ grid, const uint32_t* __restrict__ bbox0,
-                                        uint32_t* __restrict__ ubox0) {
+// Per uber cell the box of its non-zero voxels (World::ubox0, null: not wanted): brick-less
+// non-zero grid cells count whole, bricks with their non-zero box (bbox0, built before);
+// and the cell's mask for shadow rays (World::ucell): the grid cells that can stop one (bbox,
+// null: every brick might).
+__global__ void build_uber_boxes_kernel(const uint32_t* __restrict__ grid, const uint32_t* __restrict__ bbox,
+                                        const uint32_t* __restrict__ bbox0, uint32_t* __restrict__ ubox0,
+                                        unsigned long long* __restrict__ ucell) {
     const int task = blockIdx.x * blockDim.x + threadIdx.x;
     if (task >= 32 * 32 * 32) return;
     const int x = task & 31, z = (task >> 5) & 31, y = task >> 10;
-    uint32_t lo[3] = {31u, 31u, 31u}, hi[3] = {0u, 0u, 0u};
-    bool any = false;
+    uint32_t lo[3] = {31u, 31u, 31u}, hi[3] = {0u, 0u, 0u}, mask[2] = {0u, 0u};
+    bool any = false, occupied = false;
     for (int b = 0; b < 64; b++) {
         const uint32_t cx = b & 3, cz = (b >> 2) & 3, cy = b >> 4;
         const uint32_t c = __ldg(grid + (x * 4 + cx) + (z * 4 + cz) * 128 + (y * 4 + cy) * 16384);
         if (c == 0u) continue;
+        occupied = true;
+        const bool stops = (c & 1u) ? (!bbox || __ldg(bbox + (c >> 1)) != kNoOpaque) : (((c >> 1) & 0xf000u) >> 12) == 15u;
+        if (stops) mask[b >> 5] |= 1u << (b & 31);
         uint32_t l[3] = {0u, 0u, 0u}, h[3] = {7u, 7u, 7u};
-        if (c & 1u) {
+        if (bbox0 && (c & 1u)) {
             const uint32_t bb = __ldg(bbox0 + (c >> 1));
             if (bb == kNoOpaque) continue;
             for (int a = 0; a < 3; a++) { l[a] = (bb >> (3 * a)) & 7u; h[a] = (bb >> (9 + 3 * a)) & 7u; }
@@ -145,11 +156,23 @@ __global__ void build_uber_boxes_kernel(const uint32_t* __restrict__ grid, const
         for (int a = 0; a < 3; a++) { lo[a] = min(lo[a], base[a] + l[a]); hi[a] = max(hi[a], base[a] + h[a]); }
         any = true;
     }
-    uint32_t box = 0u;
-    for (int a = 0; a < 3; a++) box |= (lo[a] << (5 * a)) | (hi[a] << (15 + 5 * a));
-    ubox0[task] = any ? box : kNoOpaque;
+    if (ubox0) {
+        uint32_t box = 0u;
+        for (int a = 0; a < 3; a++) box |= (lo[a] << (5 * a)) | (hi[a] << (15 + 5 * a));
+        ubox0[task] = any ? box : kNoOpaque;
+    }
+    if (occupied && !(mask[0] | mask[1])) mask[0] = 1u;
+    ucell[task] = mask[0] | ((unsigned long long)mask[1] << 32);
 }
 
+
+// World::gbox: every grid cell with its brick's opaque box
+__global__ void build_cell_boxes_kernel(const uint32_t* __restrict__ grid, const uint32_t* __restrict__ bbox,
+                                        uint2* __restrict__ gbox) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;   // 128^3 threads
+    const uint32_t c = __ldg(grid + i);
+    gbox[i] = make_uint2(c, (c & 1u) ? __ldg(bbox + (c >> 1)) : 0u);
+}
 
 // ---- work distribution --------------------------------------------------------------------
 // VARIANT of a launch: 0 one view with area lights, 1 one view with point lights (the
@@ -429,22 +452,231 @@ __device__ __forceinline__ float phat(float3 pos, uint32_t ncode, float3 sp, uin
 // truncated) lies in the emitter cube [pos, pos + size) (GridCoordinatesFromHit /
 // Uint3CubeEquals, tools.cl:452-472). An occluded request zeroes sumOfWeights of its
 // pixel in reservoir plane C (plane 0) or H (plane 1) of its view (W follows:
-// ris.cl:79-80, 248-250). Lanes refill from the queue as soon as enough are idle. A walk
-// stops early, as occluded, once its budget cannot reach the emitter (walk_target).
-__device__ __forceinline__ void shadow_finish(const World& w, int st, const Walker& wk, float3 o, float3 L, uint32_t* plane,
-                                              uint32_t pix, uint32_t li) {
-    const float d2 = st == WALK_HIT ? wk.dist : 0.0f;
-    const uint32_t s2 = st == WALK_HIT ? wk.side : 0u;
+// ris.cl:79-80, 248-250).
+__device__ __forceinline__ bool shadow_visible(float3 o, float3 L, float d2, uint32_t s2, uint32_t pos, uint32_t size) {
     const float ns = side_sign(s2, L);
     const float hx = L.x * d2 + o.x, hy = L.y * d2 + o.y, hz = L.z * d2 + o.z;
     const uint32_t vx = f2u(hx - (s2 == 0 ? ns * 0.1f : 0.0f));
     const uint32_t vy = f2u(hy - (s2 == 1 ? ns * 0.1f : 0.0f));
     const uint32_t vz = f2u(hz - (s2 == 2 ? ns * 0.1f : 0.0f));
-    const uint32_t pos = __float_as_uint(__ldg(&w.lemit[li].w));
-    const uint32_t size = (uint32_t)__ldg(&w.lgeom[li].w);
     const uint32_t ey = pos / (1024u * 1024u), ez = (pos / 1024u) % 1024u, ex = pos % 1024u;
-    const bool inside = ex <= vx && ex + size > vx && ey <= vy && ey + size > vy && ez <= vz && ez + size > vz;
-    if (!inside) plane[(size_t)pix * 4u + 2u] = 0u;
+    return ex <= vx && ex + size > vx && ey <= vy && ey + size > vy && ez <= vz && ez + size > vz;
+}
+
+// Rays and queues of one warp of the tracer below (shared memory).
+constexpr uint32_t kCellQueue = 256, kBrickQueue = 64;   // powers of two
+constexpr int kBurst = 4;      // grid visits between two appends to the cell queue (at most 4)
+constexpr uint32_t kSolidCell = 0xFFFFFFFFu;
+struct ShadowWarp {
+    float4 a[32];                  // per lane its ray: (origin, clipped distance)
+    float4 v[32];                  // (direction, bits(view << 1 | 1 when not the request's own numbers))
+    float4 r[32];                  // (1 / direction, bits(request))
+    uint2 light[32];               // (position, size) of the emitter
+    uint2 cell[kCellQueue];        // (bits(t), packed cell | last << 21 | lane << 23)
+    uint2 walk[kBrickQueue];       // the same, of cells that have to be walked
+    float out[kBrickQueue];        // crossing behind which the ray has left their opaque voxels' box
+    uint32_t brick[kBrickQueue];   // their brick, kSolidCell for an opaque brick-less cell
+    uint32_t first[32];            // per lane: first hit of a batch, task lane << 1 | visible
+};
+
+// The tracer: each lane walks one ray's uber and grid cells (GridWalk) and appends the cells
+// that could stop it to the warp's cell queue; 32 queued cells at a time are tested by the
+// whole warp (brick-box test), the survivors' bricks queue again and 32 at a time are
+// walked by the whole warp. Queues are first in, first out, so a ray's earliest hit is the
+// first one seen; its lane takes the answer and any later tasks of it are dropped. A lane
+// is refilled from the request queue once `refill` lanes are done, after both queues
+// have been emptied (an ended walk is a miss only when none of its tasks hit).
+// Bound by instruction issue (70 % active at 960 x 540), not by memory (25 MB of DRAM reads):
+// a walker that also steps through bricks keeps 9 of 32 threads busy per instruction, since
+// some lane is always in a brick; with the bricks taken out of the walk and packed densely
+// 18 are, and a ray costs 387 warp instructions instead of 860. 1,894,052 candidate rays of
+// the 1080p frame with 65,536 emitters: 1,563 us before, 728 us now (shading's 1,801,412:
+// 1,330 and 623 us); 58,047 rays of a 333 x 187 frame, bound by the longest ray: 77 and 46
+// us. 7 blocks a SM (72 registers): 6 took 768 us, 8 (64 registers, spills) 755 us.
+// MASK: the world has cell boxes and opacity masks (else cells and voxels are read).
+template <int VARIANT, bool MASK, int MINB>
+__global__ void __launch_bounds__(128, MINB) shadow_kernel(const __grid_constant__ BatchDev bd, int countIdx, int fetchIdx,
+                                                           int planeSel) {
+    __shared__ ShadowWarp s_warp[4];
+    ShadowWarp& q = s_warp[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t n = bd.counters[countIdx];
+    uint32_t* fetch = bd.counters + fetchIdx;
+    q.first[lane] = 0xFFFFFFFFu;
+    GridWalk k;
+    const unsigned long long* ucell = bd.one.w.ucell;
+    int st = GW_IDLE;
+    bool exhausted = false;
+    uint32_t h1 = 0, n1 = 0, h2 = 0, n2 = 0;   // queue heads and lengths, the same in every lane
+    auto ray = [&](int owner) {
+        const float4 a = q.a[owner], v = q.v[owner], r = q.r[owner];
+        return ShadowRay{a.x, a.y, a.z, a.w, v.x, v.y, v.z, r.x, r.y, r.z};
+    };
+    auto view = [&](int owner) { return view_of<VARIANT>(bd, VARIANT < 2 ? 0u : __float_as_uint(q.v[owner].w) >> 1); };
+    // answer of the ray of lane `owner`: a hit at distance d on axis side, or (0, 0) for a miss
+    auto visible = [&](int owner, float d, uint32_t side) {
+        float4 a = q.a[owner], b = q.v[owner];
+        if (__float_as_uint(b.w) & 1u) {
+            const uint32_t req = __float_as_uint(q.r[owner].w);
+            a = __ldg(bd.qA + req);
+            b = __ldg(bd.qB + req);
+        }
+        const uint2 e = q.light[owner];
+        return shadow_visible(f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), d, side, e.x, e.y);
+    };
+    auto occlude = [&]() {
+        const uint32_t e = __float_as_uint(__ldg(&bd.qA[__float_as_uint(q.r[lane].w)].w));
+        const ViewDev* V = view_of<VARIANT>(bd, e >> 27);
+        reinterpret_cast<uint32_t*>(planeSel ? V->b.hA : V->b.cA)[(size_t)pix_of<VARIANT>(e) * 4u + 2u] = 0u;
+    };
+    // the first 32 tasks of the brick queue, one per lane
+    auto walk_batch = [&]() {
+        const uint32_t cnt = min(n2, 32u);
+        const uint32_t slot = (h2 + (uint32_t)lane) & (kBrickQueue - 1u);
+        const unsigned alive = __ballot_sync(0xffffffffu, st != GW_IDLE);
+        bool hit = false;
+        if ((uint32_t)lane < cnt) {
+            const uint2 rec = q.walk[slot];
+            const int owner = (int)(rec.y >> 23);
+            if ((alive >> owner) & 1u) {
+                const ShadowRay g = ray(owner);
+                const uint32_t brick = q.brick[slot];
+                const float t = __uint_as_float(rec.x);
+                float d = t * 8.0f;
+                uint32_t side = (rec.y >> 21) & 3u;
+                hit = brick == kSolidCell || brick_task<MASK>(view(owner)->w, brick, rec.y, t, q.out[slot], side, g, &d, &side);
+                if (hit) atomicMin(&q.first[owner], (uint32_t)(lane << 1) | (visible(owner, d + g.to, side) ? 1u : 0u));
+            }
+        }
+        h2 += cnt;
+        n2 -= cnt;
+        if (__any_sync(0xffffffffu, hit)) {
+            __syncwarp();
+            const uint32_t f = q.first[lane];
+            if (f != 0xFFFFFFFFu) {
+                q.first[lane] = 0xFFFFFFFFu;
+                if (!(f & 1u)) occlude();
+                st = GW_IDLE;
+            }
+        }
+        __syncwarp();
+    };
+    while (true) {
+        const unsigned idle = __ballot_sync(0xffffffffu, st == GW_IDLE);
+        if (!exhausted) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(fetch, (uint32_t)__popc(idle));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
+            const uint32_t i = base + (uint32_t)__popc(idle & below);
+            if (st == GW_IDLE && i < n) {
+                const float4 a = __ldg(bd.qA + i), b = __ldg(bd.qB + i);
+                const uint32_t vi = VARIANT < 2 ? 0u : __float_as_uint(a.w) >> 27, li = __float_as_uint(b.w);
+                const World& w = view_of<VARIANT>(bd, vi)->w;
+                q.light[lane] = make_uint2(__float_as_uint(__ldg(&w.lemit[li].w)), (uint32_t)__ldg(&w.lgeom[li].w));
+                if (VARIANT == 2) ucell = w.ucell;
+                ShadowRay g;
+                const bool walks = gw_init(k, g, ucell, a.x, a.y, a.z, b.x, b.y, b.z, 128);
+                const bool own = walks && g.ax == a.x && g.ay == a.y && g.az == a.z && g.vx == b.x && g.vy == b.y && g.vz == b.z;
+                q.a[lane] = make_float4(g.ax, g.ay, g.az, g.to);
+                q.v[lane] = make_float4(g.vx, g.vy, g.vz, __uint_as_float((vi << 1) | (own ? 0u : 1u)));
+                q.r[lane] = make_float4(g.rx, g.ry, g.rz, __uint_as_float(i));
+                st = walks ? GW_UBER : GW_END;
+            }
+            __syncwarp();
+        }
+        if (!__any_sync(0xffffffffu, st != GW_IDLE)) {
+            if (exhausted) break;
+            continue;
+        }
+        bool flush;
+        do {
+            if (st == GW_UBER) st = gw_enter(k, ray(lane), ucell);
+            // kBurst grid visits; the cells they report go to the queue together, each lane's
+            // in its order (slots by prefix sums over the lanes' counts, one ballot a bit)
+            for (int s = 0; s < bd.burst && n1 <= kCellQueue - 32u * kBurst; s += kBurst) {
+                float ct[kBurst];
+                uint32_t cp[kBurst], found = 0;
+#pragma unroll
+                for (int u = 0; u < kBurst; u++) {
+                    bool task = false;
+                    if (st == GW_GRID) {
+                        if (gw_visit(k, &task)) {
+                            ct[u] = k.t;
+                            cp[u] = (k.p & 0x1FFFFFu) | (k.last << 21);
+                            if (task) found |= 1u << u;
+                            if (!gw_step(k)) st = GW_UBER;
+                        } else {
+                            st = GW_END;
+                        }
+                    }
+                }
+                const uint32_t c = (uint32_t)__popc(found);
+                const unsigned b0 = __ballot_sync(0xffffffffu, c & 1u), b1 = __ballot_sync(0xffffffffu, c & 2u),
+                               b2 = __ballot_sync(0xffffffffu, c & 4u);
+                uint32_t slot = h1 + n1 + (uint32_t)(__popc(b0 & below) + 2 * __popc(b1 & below) + 4 * __popc(b2 & below));
+                n1 += (uint32_t)(__popc(b0) + 2 * __popc(b1) + 4 * __popc(b2));
+#pragma unroll
+                for (int u = 0; u < kBurst; u++)
+                    if (found & (1u << u))
+                        q.cell[slot++ & (kCellQueue - 1u)] = make_uint2(__float_as_uint(ct[u]), cp[u] | ((uint32_t)lane << 23));
+            }
+            const unsigned busy = __ballot_sync(0xffffffffu, st == GW_UBER || st == GW_GRID);
+            flush = busy == 0u || (!exhausted && 32 - __popc(busy) >= bd.refill);
+            __syncwarp();
+            while (n1 >= 32u || (flush && n1 > 0u)) {
+                const uint32_t cnt = min(n1, 32u);
+                const unsigned alive = __ballot_sync(0xffffffffu, st != GW_IDLE);
+                int kind = 0;
+                float out = 0.0f;
+                uint32_t brick = kSolidCell;
+                uint2 rec = make_uint2(0u, 0u);
+                if ((uint32_t)lane < cnt) {
+                    rec = q.cell[(h1 + (uint32_t)lane) & (kCellQueue - 1u)];
+                    const int owner = (int)(rec.y >> 23);
+                    if ((alive >> owner) & 1u) {
+                        const World& w = view(owner)->w;
+                        const uint32_t i = rec.y & 0x1FFFFFu;
+                        const uint2 o = MASK ? __ldg(w.gbox + i) : make_uint2(__ldg(w.grid + i), 0u);
+                        kind = grid_task<MASK>(o.x, o.y, rec.y, ray(owner), &out);
+                        if (kind == 2) brick = o.x >> 1;
+                    }
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, kind != 0);
+                if (kind != 0) {
+                    const uint32_t slot = (h2 + n2 + (uint32_t)__popc(m & below)) & (kBrickQueue - 1u);
+                    q.walk[slot] = rec;
+                    q.out[slot] = out;
+                    q.brick[slot] = brick;
+                }
+                n2 += (uint32_t)__popc(m);
+                h1 += cnt;
+                n1 -= cnt;
+                __syncwarp();
+                if (n2 >= 32u) walk_batch();
+            }
+            if (flush)
+                while (n2 > 0u) walk_batch();
+        } while (!flush);
+        // both queues are empty: a walk that ended without a hit is a miss
+        if (st == GW_END) {
+            if (!visible(lane, 0.0f, 0u)) occlude();
+            st = GW_IDLE;
+        }
+    }
+}
+
+// The same rays through the resumable walker, one cell of any level per lane and step: the
+// form that the tuning's walker options (schedule, early-out, brick cache) belong to. Lanes
+// refill from the queue as soon as enough are idle. With the early-out a walk stops, as
+// occluded, once its budget cannot reach the emitter (walk_target).
+__device__ __forceinline__ void shadow_finish(const World& w, int st, const Walker& wk, float3 o, float3 L, uint32_t* plane,
+                                              uint32_t pix, uint32_t li) {
+    const bool hit = st == WALK_HIT;
+    if (!shadow_visible(o, L, hit ? wk.dist : 0.0f, hit ? wk.side : 0u, __float_as_uint(__ldg(&w.lemit[li].w)),
+                        (uint32_t)__ldg(&w.lgeom[li].w)))
+        plane[(size_t)pix * 4u + 2u] = 0u;
 }
 
 // MINB > 0 caps registers so that MINB blocks of 128 threads fit on an SM (more warps to
@@ -454,7 +686,7 @@ __device__ __forceinline__ void shadow_finish(const World& w, int st, const Walk
 // into shared memory; with bd.bcCount set they count brick walks (calibration).
 // EARLY = 1: walks stop as occluded once their budget cannot reach the emitter.
 template <int VARIANT, int MINB, int CACHE, int EARLY>
-__global__ void __launch_bounds__(CACHE ? 512 : 128, CACHE ? 1 : MINB) shadow_kernel(const __grid_constant__ BatchDev bd,
+__global__ void __launch_bounds__(CACHE ? 512 : 128, CACHE ? 1 : MINB) shadow_walker_kernel(const __grid_constant__ BatchDev bd,
                                                                                     int countIdx, int fetchIdx,
                                                                                     int planeSel) {
     const int refill = bd.refill, burst = bd.burst, schedule = bd.schedule;
@@ -1081,18 +1313,23 @@ void launch_build_uber(const uint32_t* grid, uint8_t* uber, cudaStream_t s) {
 }
 
 void launch_build_brick_boxes(const uint32_t* bricks, const uint32_t* list, uint32_t n, uint32_t* bbox, uint32_t* bbox0,
-                              cudaStream_t s) {
+                              uint32_t* bmask, cudaStream_t s) {
     const size_t threads = (size_t)n * 32u;
     if (threads)
-        dev::build_brick_boxes_kernel<<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(bricks, list, n, bbox, bbox0);
+        dev::build_brick_boxes_kernel<<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(bricks, list, n, bbox, bbox0, bmask);
 }
 
 void launch_commit_bricks(const uint32_t* list, const uint32_t* voxels, uint32_t n, uint32_t* bricks, cudaStream_t s) {
     if (n) dev::commit_bricks_kernel<<<n, 128, 0, s>>>(list, voxels, bricks);
 }
 
-void launch_build_uber_boxes(const uint32_t* grid, const uint32_t* bbox0, uint32_t* ubox0, cudaStream_t s) {
-    dev::build_uber_boxes_kernel<<<(32 * 32 * 32 + 255) / 256, 256, 0, s>>>(grid, bbox0, ubox0);
+void launch_build_uber_boxes(const uint32_t* grid, const uint32_t* bbox, const uint32_t* bbox0, uint32_t* ubox0,
+                             unsigned long long* ucell, cudaStream_t s) {
+    dev::build_uber_boxes_kernel<<<(32 * 32 * 32 + 63) / 64, 64, 0, s>>>(grid, bbox, bbox0, ubox0, ucell);
+}
+
+void launch_build_cell_boxes(const uint32_t* grid, const uint32_t* bbox, uint2* gbox, cudaStream_t s) {
+    dev::build_cell_boxes_kernel<<<128 * 128 * 128 / 256, 256, 0, s>>>(grid, bbox, gbox);
 }
 
 void launch_path_trace(const BatchDev& bd, cudaStream_t s) {
@@ -1106,18 +1343,19 @@ void launch_batch_albedo(const BatchDev& bd, int variant, cudaStream_t s) {
     else launch_tiles(dev::albedo_kernel<0>, bd, kCtrAlbedo, s, K_ALBEDO);
 }
 
-template <int VARIANT, int MINB, int EARLY>
-static void launch_shadow_k(const BatchDev& bd, int countIdx, int planeSel, cudaStream_t s) {
-    const size_t rb = resident_blocks((const void*)dev::shadow_kernel<VARIANT, MINB, 0, EARLY>, 128);
+constexpr int kShadowMinBlocks = 7;   // of shadow_kernel: 728 us against 768 at 6 and 755 at 8 (see there)
+template <class K>
+static void launch_shadow_rays(K kernel, const BatchDev& bd, int countIdx, int planeSel, cudaStream_t s) {
+    const size_t rb = resident_blocks((const void*)kernel, 128);
     const unsigned nb = (unsigned)std::max<size_t>(1, std::min<size_t>(rb, ((size_t)bd.totalPixels + 127) / 128));
     Timed tm(bd, planeSel ? K_SHADOW_SHADE : K_SHADOW_CAND, s);
-    dev::shadow_kernel<VARIANT, MINB, 0, EARLY><<<nb, 128, 0, s>>>(bd, countIdx, countIdx + 1, planeSel);
+    kernel<<<nb, 128, 0, s>>>(bd, countIdx, countIdx + 1, planeSel);
 }
 // shared memory of the brick-cache variant: 2^log2 keys and 2^(log2 - 1) masks of 64 bytes
 size_t brick_cache_smem(int log2) { return log2 > 0 ? ((size_t)4 << log2) + ((size_t)64 << (log2 - 1)) : 0; }
 template <int EARLY>
 static void launch_shadow_cached(const BatchDev& bd, int countIdx, int planeSel, cudaStream_t s) {
-    const void* fn = (const void*)dev::shadow_kernel<0, 0, 1, EARLY>;
+    const void* fn = (const void*)dev::shadow_walker_kernel<0, 0, 1, EARLY>;
     const size_t sm = brick_cache_smem(bd.bcLog2);
     if (sm > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     int per = 0;
@@ -1125,7 +1363,7 @@ static void launch_shadow_cached(const BatchDev& bd, int countIdx, int planeSel,
     const size_t rb = (size_t)std::max(per, 1) * (size_t)sm_count();
     const unsigned nb = (unsigned)std::max<size_t>(1, std::min<size_t>(rb, ((size_t)bd.totalPixels + 511) / 512));
     Timed tm(bd, planeSel ? K_SHADOW_SHADE : K_SHADOW_CAND, s);
-    dev::shadow_kernel<0, 0, 1, EARLY><<<nb, 512, sm, s>>>(bd, countIdx, countIdx + 1, planeSel);
+    dev::shadow_walker_kernel<0, 0, 1, EARLY><<<nb, 512, sm, s>>>(bd, countIdx, countIdx + 1, planeSel);
 }
 template <int VARIANT>
 static void launch_shadow(const BatchDev& bd, int countIdx, int planeSel, cudaStream_t s) {
@@ -1133,12 +1371,18 @@ static void launch_shadow(const BatchDev& bd, int countIdx, int planeSel, cudaSt
     if (VARIANT < 2 && (bd.bcLog2 > 0 || bd.bcCount)) {
         if (early) launch_shadow_cached<1>(bd, countIdx, planeSel, s);
         else launch_shadow_cached<0>(bd, countIdx, planeSel, s);
-    } else if (bd.occupancy) {
-        if (early) launch_shadow_k<VARIANT, 8, 1>(bd, countIdx, planeSel, s);
-        else launch_shadow_k<VARIANT, 8, 0>(bd, countIdx, planeSel, s);
+    } else if (early) {
+        launch_shadow_rays(dev::shadow_walker_kernel<VARIANT, 8, 0, 1>, bd, countIdx, planeSel, s);
+    } else if (bd.schedule) {
+        launch_shadow_rays(dev::shadow_walker_kernel<VARIANT, 8, 0, 0>, bd, countIdx, planeSel, s);
     } else {
-        if (early) launch_shadow_k<VARIANT, 0, 1>(bd, countIdx, planeSel, s);
-        else launch_shadow_k<VARIANT, 0, 0>(bd, countIdx, planeSel, s);
+        if constexpr (VARIANT == 0) {
+            if (!bd.one.w.bmask) {   // a caller's bricks (vxr_render_frame_noalloc): no masks
+                launch_shadow_rays(dev::shadow_kernel<0, false, kShadowMinBlocks>, bd, countIdx, planeSel, s);
+                return;
+            }
+        }
+        launch_shadow_rays(dev::shadow_kernel<VARIANT, true, kShadowMinBlocks>, bd, countIdx, planeSel, s);
     }
 }
 template <int VARIANT, bool LEARNED>

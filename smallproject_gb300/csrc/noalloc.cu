@@ -46,6 +46,7 @@ static_assert(kScratchBytes == VXR_NOALLOC_SCRATCH_BYTES, "scratch size must mat
 static_assert(kOffSeed % 256 == 0 && kOffCA % 256 == 0 && kOffUber % 256 == 0 && kOffGeom % 256 == 0 &&
                   kOffHits % 256 == 0 && kOffQA % 256 == 0 && kOffErr % 256 == 0,
               "scratch regions must stay 256-byte aligned");
+static_assert(16 * kMaxLights >= 8 * 32 * 32 * 32, "the uber cells' masks must fit the region of the widened lights");
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -136,6 +137,10 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
         vxr::launch_build_light_table(raw, nlights, geom, emit, st);
     }
     vxr::launch_build_uber(grid, s + kOffUber, st);
+    // the uber cells' masks take the place of the widened lights, which only the light
+    // table's kernel reads
+    unsigned long long* ucell = (unsigned long long*)raw;
+    vxr::launch_build_uber_boxes(grid, nullptr, nullptr, nullptr, ucell, st);
     CUN(cudaGetLastError(), "world kernels");
 
     vxr::dev::World w;
@@ -145,6 +150,7 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     w.bbox = nullptr;   // no room for brick boxes: rays walk every brick they meet
     w.bbox0 = nullptr;
     w.ubox0 = nullptr;
+    w.ucell = ucell;
     w.lgeom = geom;
     w.lemit = emit;
     w.nlights = nlights;

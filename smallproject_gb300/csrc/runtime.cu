@@ -35,7 +35,10 @@ void release_device_world(World& w) {
     cudaFree(d->uber);
     cudaFree(d->bricks);
     cudaFree(d->bbox);
+    cudaFree(d->bmask);
     cudaFree(d->ubox0);
+    cudaFree(d->ucell);
+    cudaFree(d->gbox);
     cudaFree(d->stageDev);
     cudaFreeHost(d->stageHost);
     cudaFree(d->lraw);
@@ -71,6 +74,8 @@ static int upload(World& w) {
     if (!d.grid) CU(cudaMalloc(&d.grid, kGridSize * sizeof(uint32_t)), "cudaMalloc(grid)");
     if (!d.uber) CU(cudaMalloc(&d.uber, 32 * 32 * 32), "cudaMalloc(uber)");
     if (!d.ubox0) CU(cudaMalloc(&d.ubox0, 32 * 32 * 32 * sizeof(uint32_t)), "cudaMalloc(uber boxes)");
+    if (!d.ucell) CU(cudaMalloc(&d.ucell, 32 * 32 * 32 * sizeof(unsigned long long)), "cudaMalloc(uber cells)");
+    if (!d.gbox) CU(cudaMalloc(&d.gbox, kGridSize * sizeof(uint2)), "cudaMalloc(cell boxes)");
     uint32_t sent = 0;
     if (full) {
         if (w.brickHigh > d.cap || !d.bricks) {
@@ -79,10 +84,13 @@ static int upload(World& w) {
             cudaFree(d.bricks);
             cudaFree(d.bbox);
             d.bricks = nullptr;
+            cudaFree(d.bmask);
             d.bbox = nullptr;
+            d.bmask = nullptr;
             d.cap = 0;
             CU(cudaMalloc(&d.bricks, (size_t)cap * kBrick * sizeof(uint32_t)), "cudaMalloc(bricks)");
             CU(cudaMalloc(&d.bbox, (size_t)cap * 2u * sizeof(uint32_t)), "cudaMalloc(brick boxes)");
+            CU(cudaMalloc(&d.bmask, (size_t)cap * 16u * sizeof(uint32_t)), "cudaMalloc(brick masks)");
             d.cap = cap;
         }
         d.bbox0 = d.bbox + d.cap;
@@ -90,7 +98,7 @@ static int upload(World& w) {
         if (w.brickHigh)
             CU(cudaMemcpy(d.bricks, w.bricks.data(), (size_t)w.brickHigh * kBrick * sizeof(uint32_t), cudaMemcpyHostToDevice),
                "upload bricks");
-        launch_build_brick_boxes(d.bricks, nullptr, w.brickHigh, d.bbox, d.bbox0, 0);
+        launch_build_brick_boxes(d.bricks, nullptr, w.brickHigh, d.bbox, d.bbox0, d.bmask, 0);
         sent = w.brickHigh;
     } else if (w.dirtyCount) {
         if (w.dirtyCount > d.stageCap) {
@@ -125,7 +133,7 @@ static int upload(World& w) {
             const size_t bytes = (voxOff + (size_t)k * kBrick) * sizeof(uint32_t);
             CU(cudaMemcpy(d.stageDev, d.stageHost, bytes, cudaMemcpyHostToDevice), "commit bricks");
             launch_commit_bricks(d.stageDev, d.stageDev + voxOff, k, d.bricks, 0);
-            launch_build_brick_boxes(d.bricks, d.stageDev, k, d.bbox, d.bbox0, 0);
+            launch_build_brick_boxes(d.bricks, d.stageDev, k, d.bbox, d.bbox0, d.bmask, 0);
         }
     }
     if (full || w.gridDirty) {
@@ -144,7 +152,10 @@ static int upload(World& w) {
         }
         launch_build_uber(d.grid, d.uber, 0);
     }
-    if (full || w.gridDirty || sent) launch_build_uber_boxes(d.grid, d.bbox0, d.ubox0, 0);
+    if (full || w.gridDirty || sent) {
+        launch_build_uber_boxes(d.grid, d.bbox, d.bbox0, d.ubox0, d.ucell, 0);
+        launch_build_cell_boxes(d.grid, d.bbox, d.gbox, 0);
+    }
     if (full || d.lightVersion != w.lightVersion || d.lightMoveVersion != w.lightMoveVersion) {
         const uint32_t nl = (uint32_t)w.lights.size();
         const size_t need = std::max<uint32_t>(nl, 1u);
@@ -207,6 +218,9 @@ vxr::dev::World dev_world(vxr_view* v) {
     w.bbox = d.bbox;
     w.bbox0 = d.bbox0;
     w.ubox0 = d.ubox0;
+    w.ucell = d.ucell;
+    w.bmask = d.bmask;
+    w.gbox = d.gbox;
     w.lgeom = d.lgeom;
     w.lemit = d.lemit;
     w.nlights = d.nl;
@@ -460,8 +474,8 @@ int vxr_world_pending(const vxr_world* w, uint32_t* dirty_bricks, int* grid_chan
 int vxr_world_device_bytes(const vxr_world* w, uint64_t* bytes) {
     VXR_CHECK_ARG(w && bytes, "vxr_world_device_bytes: null argument");
     const vxr::DeviceWorld* d = w->w.dev;
-    // grid, uber grid and its boxes, bricks and their boxes, light tables
-    *bytes = d ? (uint64_t)(vxr::kGridSize * 4 + 32768 + 32768 * 4 + (uint64_t)d->cap * (vxr::kBrick * 4 + 8) +
+    // grid and its boxes, uber grid, its boxes and masks, bricks, their boxes and masks, light tables
+    *bytes = d ? (uint64_t)(vxr::kGridSize * 12 + 32768 + 32768 * 4 + 32768 * 8 + (uint64_t)d->cap * (vxr::kBrick * 4 + 8 + 64) +
                             (uint64_t)d->stageCap * (vxr::kBrick + 1) * 4 + d->lcap * 48)
                : 0;
     return VXR_OK;

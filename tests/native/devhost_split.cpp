@@ -1,0 +1,73 @@
+// devhost_split.cpp - the split shadow DDA (GridWalk, grid_task, brick_task in device.cuh)
+// run on the host, one ray at a time, tasks in visiting order, as the tracer's queues keep
+// them. Test infrastructure only.
+#include "devhost.cpp"
+
+extern "C" {
+
+// As dh_shadow (the resumable walker): 1 when the visibility test passes. deferred: every
+// task is finished after the walk has ended (as when a warp's queue is emptied late), else
+// at once. stats[4]: uber cells entered, grid cells visited, tasks, bricks walked.
+int dh_shadow_split(const uint32_t* grid, const uint32_t* bricks, const uint32_t* bbox, const uint32_t* ucell,
+                    const uint32_t* bmask, const float* O, const float* D, uint32_t pos, uint32_t size, int steps, int deferred, int* stats,
+                    float* dist, uint32_t* side) {
+    World w = make_world(grid, nullptr, bricks);
+    w.bmask = bmask;
+    struct Task { float t; uint32_t cell, last; };
+    static Task tasks[4096];
+    int n = 0, done = 0;
+    GridWalk k;
+    ShadowRay g;
+    const auto* masks = reinterpret_cast<const unsigned long long*>(ucell);
+    int st = gw_init(k, g, masks, O[0], O[1], O[2], D[0], D[1], D[2], steps) ? GW_UBER : GW_END;
+    bool hit = false;
+    float d2 = 0.0f;
+    uint32_t s2 = 0;
+    auto finish = [&]() {
+        for (; done < n && !hit; done++) {
+            const Task& q = tasks[done];
+            const uint32_t o = grid[q.cell & 0x1FFFFFu];
+            float out;
+            const int kind = bbox ? grid_task<true>(o, (o & 1u) ? bbox[o >> 1] : 0u, q.cell, g, &out)
+                                  : grid_task<false>(o, 0u, q.cell, g, &out);
+            s2 = q.last;
+            if (kind == 1) { hit = true; d2 = q.t * 8.0f; }
+            if (kind == 2) {
+                stats[3]++;
+                const auto walk = bmask ? brick_task<true> : brick_task<false>;
+                hit = walk(w, o >> 1, q.cell, q.t, out, q.last, g, &d2, &s2);
+            }
+        }
+    };
+    while (st != GW_END && !hit) {
+        if (st == GW_UBER) {
+            st = gw_enter(k, g, masks);
+            if (st == GW_GRID) stats[0]++;
+            continue;
+        }
+        bool task = false;
+        if (!gw_visit(k, &task)) { st = GW_END; continue; }
+        stats[1]++;
+        if (task) {
+            stats[2]++;
+            tasks[n++] = Task{k.t, k.p & 0x1FFFFFu, k.last};
+            if (!deferred) finish();
+        }
+        if (!gw_step(k)) st = GW_UBER;
+    }
+    finish();
+    d2 = hit ? d2 + g.to : 0.0f;
+    s2 = hit ? s2 : 0u;
+    *dist = d2;
+    *side = hit ? s2 : 3u;
+    const float3 L = f3(D[0], D[1], D[2]);
+    const float ns = side_sign(s2, L);
+    const float hx = L.x * d2 + O[0], hy = L.y * d2 + O[1], hz = L.z * d2 + O[2];
+    const uint32_t vx = f2u(hx - (s2 == 0 ? ns * 0.1f : 0.0f));
+    const uint32_t vy = f2u(hy - (s2 == 1 ? ns * 0.1f : 0.0f));
+    const uint32_t vz = f2u(hz - (s2 == 2 ? ns * 0.1f : 0.0f));
+    const uint32_t ey = pos / (1024u * 1024u), ez = (pos / 1024u) % 1024u, ex = pos % 1024u;
+    return ex <= vx && ex + size > vx && ey <= vy && ey + size > vy && ez <= vz && ez + size > vz;
+}
+
+}  // extern "C"

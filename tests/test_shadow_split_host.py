@@ -1,0 +1,122 @@
+"""The split shadow DDA (GridWalk and its tasks, device.cuh) compiled for the CPU, against the
+resumable walker: the same status, distance bits, side and visibility for every ray, tasks
+finished at once or after the walk, with and without brick boxes and masks."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+from oracle import binding as ob
+from test_device_code_host import _candidate_shadow_rays, _f3, _rays, _surface_rays, brick_boxes, dh  # noqa: F401
+
+NATIVE = os.path.join(ROOT, "tests", "native")
+
+
+@pytest.fixture(scope="module")
+def split(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("split") / "libsplit.so")
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-fno-fast-math", "-w", "-I" + cuda,
+                    "-I" + os.path.join(ROOT, "smallproject_gb300", "csrc"), os.path.join(NATIVE, "devhost_split.cpp"), "-o", so],
+                   check=True)
+    lib = C.CDLL(so)
+    P, F = C.c_void_p, C.POINTER(C.c_float)
+    lib.dh_shadow_split.argtypes = [P, P, P, P, P, F, F, C.c_uint32, C.c_uint32, C.c_int, C.c_int, C.POINTER(C.c_int), F,
+                                    C.POINTER(C.c_uint32)]
+    return lib
+
+
+def uber_cells(grid, bricks, boxes):
+    """World::ucell as the GPU builds it (build_uber_boxes_kernel); boxes None: every brick
+    counts as one that can stop a ray."""
+    g = grid.reshape(128, 128, 128)                                    # [y, z, x]
+    brick = (g & 1) == 1
+    stops = ~brick & ((((g >> 1) >> 12) & 15) == 15)
+    stops[brick] = True if boxes is None else boxes[g[brick] >> 1] != 0xFFFFFFFF
+    out = np.zeros((32, 32, 32, 2), np.uint32)                         # [uy, uz, ux]
+    for b in range(64):
+        s = stops[b >> 4::4, (b >> 2) & 3::4, b & 3::4].astype(np.uint32)
+        out[..., b >> 5] |= s << np.uint32(b & 31)
+    occupied = (g != 0).reshape(32, 4, 32, 4, 32, 4).any(axis=(1, 3, 5))
+    out[..., 0] |= (occupied & ~out.any(axis=-1)).astype(np.uint32)
+    return np.ascontiguousarray(out.reshape(-1, 2))
+
+
+def brick_masks(bricks):
+    """World::bmask as the GPU builds it (build_brick_boxes_kernel)."""
+    op = ((bricks.reshape(-1, 16, 32) >> 12) & 15) == 15
+    return (op.astype(np.uint32) << np.arange(32, dtype=np.uint32)).sum(axis=2, dtype=np.uint32)
+
+
+def _compare(dh, split, wa, O, D, pos, size, stepss):  # noqa: F811
+    boxes, masks = brick_boxes(wa.bricks), brick_masks(wa.bricks)
+    P = lambda a: a.ctypes.data  # noqa: E731
+    hits = visible = 0
+    stats = (C.c_int * 4)()
+    for bx, mk in ((boxes, masks), (None, None)):
+        uc = uber_cells(wa.grid, wa.bricks, bx)
+        for i in range(len(O)):
+            o, d, steps = _f3(O[i]), _f3(D[i]), int(stepss[i])
+            da, sa, nv = C.c_float(0), C.c_uint32(0), C.c_int(0)
+            st = dh.dh_walk_skip(P(wa.grid), P(wa.uber), P(wa.bricks), P(boxes), o, d, steps, C.byref(da), C.byref(sa),
+                                 C.byref(nv))
+            want = dh.dh_shadow(P(wa.grid), P(wa.uber), P(wa.bricks), P(boxes), o, d, int(pos[i]), int(size[i]), 0,
+                                C.byref(nv)) if steps == 128 else None
+            for deferred in (0, 1):
+                db, sb = C.c_float(0), C.c_uint32(0)
+                got = split.dh_shadow_split(P(wa.grid), P(wa.bricks), P(bx) if bx is not None else None, P(uc),
+                                            P(mk) if mk is not None else None, o, d, int(pos[i]), int(size[i]), steps, deferred, stats, C.byref(db), C.byref(sb))
+                assert (sb.value != 3) == (st == 1), (i, O[i], D[i], steps)
+                assert np.float32(da.value).view(np.uint32) == np.float32(db.value).view(np.uint32), (i, O[i], D[i])
+                assert st != 1 or sa.value == sb.value, (i, O[i], D[i])
+                assert want is None or got == want, (i, O[i], D[i])
+            hits += st == 1
+            visible += bool(want)
+    return hits, visible, list(stats)
+
+
+def test_split_walk_matches_walker(dh, split, world0_arrays):  # noqa: F811
+    """Rays through and past the map, axis-aligned ones among them, rays leaving the terrain,
+    budgets from 1 to endless; the emitter is drawn at random (the hit decides) and a NaN
+    direction ends as the walker's does."""
+    wa = world0_arrays
+    o1, d1, rng = _rays(2500, 77)
+    o2, d2, _ = _surface_rays(wa, 2500, 78)
+    o3 = np.tile(np.float32([[128.5, 200.5, 128.5]]), (3, 1))
+    d3 = np.float32([[0, -1, 0], [np.nan, np.nan, np.nan], [np.inf, 0, 0]])
+    O, D = np.concatenate([o1, o2, o3]), np.concatenate([d1, d2, d3])
+    steps = rng.choice([128, 128, 128, 5000, 9, 5, 4, 1], len(O))
+    li = rng.integers(0, len(wa.lights), len(O))
+    hits, _, _ = _compare(dh, split, wa, O, D, wa.lights["position"][li], wa.lights["size"][li], steps)
+    assert hits > 500
+
+
+@pytest.mark.parametrize("point", [False, True])
+def test_split_walk_matches_walker_on_candidate_rays(dh, split, world0_arrays, point):  # noqa: F811
+    wa = world0_arrays
+    O, D, LI = _candidate_shadow_rays(wa, wa.lights, 96, 54,
+                                      lambda f: ((128.0 + 40.0 * f, 170.0, -60.0 + 30.0 * f), (128.0, 100.0, 128.0)), point)
+    hits, visible, _ = _compare(dh, split, wa, O, D, wa.lights["position"][LI], wa.lights["size"][LI], np.full(len(O), 128))
+    assert hits > 500 and visible > 100
+
+
+def test_split_walk_finds_solid_cells(dh, split):  # noqa: F811
+    """Brick-less cells: opaque ones stop a ray at their entry point, translucent ones do not
+    (nor does an uber cell that holds nothing else, but its cells still cost budget)."""
+    import smallproject_gb300 as vx
+    w = vx.World()
+    rng = np.random.default_rng(5)
+    for b in rng.integers(0, 16, (160, 3)):
+        w.add_brick(int(b[0]), int(b[1]), int(b[2]), 0xF123 if rng.random() < 0.5 else 0x8123)
+    for b in rng.integers(0, 128, (400, 3)):
+        w.set(int(b[0]), int(b[1]), int(b[2]), 0xFFFF if rng.random() < 0.7 else 0x7ABC)
+    g, bricks, lights = w.arrays()
+    wa = ob.WorldArrays(g, bricks, lights)
+    O, D, rng = _rays(2500, 6, lo=-40.0, hi=170.0, inside=(0.0, 128.0))
+    n = len(O)
+    hits, _, _ = _compare(dh, split, wa, O, D, rng.integers(0, 1 << 30, n), rng.choice([1, 8], n),
+                          rng.choice([128, 30, 9], n))
+    assert hits > 300
