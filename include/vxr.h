@@ -500,8 +500,8 @@ typedef struct vxr_tuning {
     uint32_t persistent;           /* pixel stages: 1 = resident blocks pull tiles from a queue, 0 = one block per tile */
     uint32_t shadow_refill;        /* shadow tracer: idle lanes of a warp (1..32) that trigger a refill from the queue */
     uint32_t shadow_burst;         /* shadow tracer: grid-cell visits per lane between refill checks (1..64, in steps of 4) */
-    uint32_t list_blocks_per_sm;   /* hit-list kernels (candidates, temporal, shading requests): blocks per SM (1..64) */
-    uint32_t occupancy;            /* 1: candidate kernel capped in registers for more warps per SM */
+    uint32_t list_blocks_per_sm;   /* hit-list kernels (temporal, shading requests): blocks per SM (1..64) */
+    uint32_t occupancy;            /* 0 or 1; no effect (kernels are built at the register count that measured fastest) */
     /* the next three belong to the tracer that walks a ray's cells of all levels in one
        lane; any of them set selects it (the default tracer walks bricks by whole warps) */
     uint32_t shadow_schedule;      /* shadow tracer: 0 every lane steps each round, 1 only the lanes at the DDA level most lanes are at */

@@ -403,47 +403,6 @@ __global__ void __launch_bounds__(256) compact_hits_kernel(const __grid_constant
     }
 }
 
-// ---- target function (phat.cl:2-41) ------------------------------------------------------
-// length(brdf * Le/pi * cos(theta) * cos(theta_l) * size^2 / d^2), NaN/Inf -> 0.
-// The zero cases are decided from signs before any division: N is an axis normal, so
-// dot(N, L) = sN * L[side] and sign(L[a]) = sign(R[a]); a non-positive cosine makes the
-// product exactly (+/-)0, whose length is +0.
-template <bool POINT>
-__device__ __forceinline__ float3 phat_full(float3 pos, uint32_t ncode, float3 sp, uint32_t nside, float nsign,
-                                            float3 brdf, float4 em, float size, bool* zero) {
-    const float3 R = sub(pos, sp);
-    *zero = true;
-    if (!(nsign * comp(R, nside) > 0.0f)) return f3(0.0f, 0.0f, 0.0f);
-    float lsign = 0.0f;
-    uint32_t laxis = 0;
-    if (!POINT) {
-        if (ncode >= 6) return f3(0.0f, 0.0f, 0.0f);
-        laxis = ncode % 3;
-        lsign = ncode < 3 ? 1.0f : -1.0f;
-        if (!(-(lsign * comp(R, laxis)) > 0.0f)) return f3(0.0f, 0.0f, 0.0f);
-    }
-    *zero = false;
-    const float dd = dot3(R, R);
-    const float inv = 1.0f / sqrtf(dd);
-    const float3 L = mul(R, inv);
-    const float ndotl = fmaxf(nsign * comp(L, nside), 0.0f);
-    const float distsq = fmaxf(1e-5f, dd);
-    const float area = size * size;
-    const float nldotl = POINT ? 1.0f : fmaxf(-(lsign * comp(L, laxis)), 0.0f);
-    const float solid = (nldotl * area) / distsq;
-    return f3(((brdf.x * em.x) * ndotl) * solid, ((brdf.y * em.y) * ndotl) * solid, ((brdf.z * em.z) * ndotl) * solid);
-}
-template <bool POINT>
-__device__ __forceinline__ float phat(float3 pos, uint32_t ncode, float3 sp, uint32_t nside, float nsign, float3 brdf,
-                                      float4 em, float size) {
-    bool zero;
-    const float3 c = phat_full<POINT>(pos, ncode, sp, nside, nsign, brdf, em, size, &zero);
-    if (zero) return 0.0f;
-    const float r = sqrtf(dot3(c, c));
-    if (isnan(r) || isinf(r)) return 0.0f;
-    return r;
-}
-
 // ---- visibility (isLightOccluded, ris.cl:1-17) -----------------------------------------
 // Persistent shadow tracer over the batch's request queue. Requests:
 // qA = (origin, bits(view << 27 | pixel)), qB = (dir, bits(light)). Budget GRIDWIDTH = 128
@@ -777,6 +736,9 @@ __global__ void __launch_bounds__(CACHE ? 512 : 128, CACHE ? 1 : MINB) shadow_wa
 // Over the hit list. Ends with AdjustWeight(res, res.pHat) (implied by the stored
 // sumW, pHat, M) and a shadow-ray request for the selected sample when sumW > 0 (when
 // sumW == 0 the discard of ris.cl:79-80 changes nothing).
+// Bound by instruction issue (80 % active, the ALU pipe 66 %): area_candidate's branch-free
+// roots and quotients take a candidate from 761 to 497 warp instructions, 1,894,057 hit
+// pixels x 32 candidates from 1,563 to 914 us, x 4 learned ones from 281 to 166 us.
 // LEARNED: the light index and its source pdf p come from the learned proposal (drawn
 // by the inference kernel) instead of GenerateLightCandidate's uniform 1 / N.
 template <bool POINT, bool LEARNED>
@@ -821,16 +783,21 @@ __device__ __forceinline__ void ris_item(const BatchDev& bd, const ViewDev* V, u
         const float4 lg = __ldg(w.lgeom + li);
         const float4 le = __ldg(w.lemit + li);
         float3 pos;
-        float inv;
+        float inv, ph;
         uint32_t nc;
         if (POINT) {
             pos = f3(lg.x, lg.y, lg.z);
             inv = 1.0f;
             nc = 6;
+            ph = phat<true>(pos, nc, sp, side, nsign, brdf, le, lg.w) * inv;
         } else {
-            pos = sample_area_light(lg, spo, seed, &inv, &nc);
+            const uint32_t seed0 = seed;
+            if (!area_candidate(lg, le, sp, spo, side, nsign, brdf, seed, &ph, &pos, &inv, &nc)) {
+                seed = seed0;
+                pos = sample_area_light(lg, spo, seed, &inv, &nc);
+                ph = phat<false>(pos, nc, sp, side, nsign, brdf, le, lg.w) * inv;
+            }
         }
-        const float ph = phat<POINT>(pos, nc, sp, side, nsign, brdf, le, lg.w) * inv;
         res_update(res, pow2 ? ph * nLf : ph / p, ph, (uint32_t)li, rnd(seed), pos, inv, nc);
     }
     if (k.ncand > 0 && res.sumW > 0.0f) {
@@ -1277,7 +1244,6 @@ void apply_tuning(BatchDev& bd, const Tuning& tu) {
     bd.refill = tu.refill;
     bd.burst = tu.burst;
     bd.listPerSm = tu.listPerSm;
-    bd.occupancy = tu.occupancy;
     bd.schedule = tu.schedule;
     bd.earlyOut = tu.earlyOut;
 }
@@ -1385,11 +1351,16 @@ static void launch_shadow(const BatchDev& bd, int countIdx, int planeSel, cudaSt
         launch_shadow_rays(dev::shadow_kernel<VARIANT, true, kShadowMinBlocks>, bd, countIdx, planeSel, s);
     }
 }
+// 64 registers: at 1080p 914 us against 937 (7 blocks a SM), 988 (6) and 987 (5)
+constexpr int kRisMinBlocks = 8;
+// A block per 128 pixels of the batch, those past the hit list's end leaving at once: a warp's
+// candidates take long enough that the block scheduler balances them better than resident
+// blocks striding over the list (1080p, 7 blocks a SM: 937 us against 1,005).
 template <int VARIANT, bool LEARNED>
-static void launch_ris(const BatchDev& bd, unsigned nb, cudaStream_t s) {
+static void launch_ris(const BatchDev& bd, cudaStream_t s) {
+    const unsigned nb = (unsigned)(((size_t)bd.totalPixels + 127) / 128);
     Timed tm(bd, K_RIS, s);
-    if (bd.occupancy) dev::ris_kernel<VARIANT, LEARNED, 7><<<nb, 128, 0, s>>>(bd);
-    else dev::ris_kernel<VARIANT, LEARNED, 0><<<nb, 128, 0, s>>>(bd);
+    dev::ris_kernel<VARIANT, LEARNED, kRisMinBlocks><<<nb, 128, 0, s>>>(bd);
 }
 
 template <int VARIANT>
@@ -1436,11 +1407,11 @@ static void candidates_v(const BatchDev& bd, const LearnedHook* learned, cudaStr
                 }
                 prop::launch_infer(ia, (uint32_t)n, s);
             }
-            launch_ris<VARIANT, true>(lb, nb, s);
+            launch_ris<VARIANT, true>(lb, s);
             learnedDone = true;
         }
     }
-    if (!learnedDone) launch_ris<VARIANT, false>(bd, nb, s);
+    if (!learnedDone) launch_ris<VARIANT, false>(bd, s);
     launch_shadow<VARIANT < 2 ? 0 : 2>(bd, kCtrQ1, 0, s);
     if (tail && tail != s) {
         cudaEventRecord(ev, s);

@@ -89,7 +89,6 @@ struct BatchDev {
     int refill = 8;                       // shadow tracer: idle lanes of a warp that trigger a refill
     int burst = 4;                        // shadow tracer: cell visits per lane between refill checks
     int listPerSm = 16;                   // blocks per SM of the hit-list kernels
-    int occupancy = 0;                    // 1: register-capped shadow / RIS kernels (more warps per SM)
     int schedule = 0;                     // shadow tracer: 1 = one DDA level per round (the majority's)
     int earlyOut = 0;                     // shadow tracer: stop a walk once its budget cannot reach the emitter
     // shadow tracer's brick cache (single views): the table (global; each CTA copies it
@@ -114,7 +113,7 @@ struct Tuning {
     int refill = 8;
     int burst = 4;
     int listPerSm = 16;
-    int occupancy = 0;
+    int occupancy = 0;                    // kept for vxr_view_get_tuning: no kernel has two register counts any more
     int schedule = 0;
     int earlyOut = 0;
     int brickCache = 0;

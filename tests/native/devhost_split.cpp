@@ -1,6 +1,6 @@
 // devhost_split.cpp - the split shadow DDA (GridWalk, grid_task, brick_task in device.cuh)
 // run on the host, one ray at a time, tasks in visiting order, as the tracer's queues keep
-// them. Test infrastructure only.
+// them; and the one-call area-light candidate. Test infrastructure only.
 #include "devhost.cpp"
 
 extern "C" {
@@ -68,6 +68,31 @@ int dh_shadow_split(const uint32_t* grid, const uint32_t* bricks, const uint32_t
     const uint32_t vz = f2u(hz - (s2 == 2 ? ns * 0.1f : 0.0f));
     const uint32_t ey = pos / (1024u * 1024u), ez = (pos / 1024u) % 1024u, ex = pos % 1024u;
     return ex <= vx && ex + size > vx && ey <= vy && ey + size > vy && ez <= vz && ez + size > vz;
+}
+
+// An area-light candidate: one call (area_candidate) and the two functions it stands for.
+// in: light centre, size, emission rgb, shading point, offset point, normal sign, albedo/pi rgb;
+// out[which]: ph, seed bits, point xyz, weight, face bits. Returns area_candidate's answer.
+int dh_area_candidate(const float* in, uint32_t side, uint32_t seed, float* out) {
+    const float4 g = make_float4(in[0], in[1], in[2], in[3]), em = make_float4(in[4], in[5], in[6], 0.0f);
+    const float3 sp = f3(in[7], in[8], in[9]), spo = f3(in[10], in[11], in[12]), brdf = f3(in[14], in[15], in[16]);
+    int ok = 0;
+    for (int which = 0; which < 2; which++) {
+        uint32_t s = seed, face = 9;
+        float3 pos = f3(0.0f, 0.0f, 0.0f);
+        float ph = 0.0f, inv = 0.0f;
+        if (which == 0) {
+            ok = area_candidate(g, em, sp, spo, side, in[13], brdf, s, &ph, &pos, &inv, &face);
+        } else {
+            pos = sample_area_light(g, spo, s, &inv, &face);
+            ph = phat<false>(pos, face, sp, side, in[13], brdf, em, g.w) * inv;
+        }
+        float* o = out + 7 * which;
+        o[0] = ph; o[2] = pos.x; o[3] = pos.y; o[4] = pos.z; o[5] = inv;
+        std::memcpy(o + 1, &s, 4);
+        std::memcpy(o + 6, &face, 4);
+    }
+    return ok;
 }
 
 }  // extern "C"

@@ -1,6 +1,7 @@
 """The split shadow DDA (GridWalk and its tasks, device.cuh) compiled for the CPU, against the
 resumable walker: the same status, distance bits, side and visibility for every ray, tasks
-finished at once or after the walk, with and without brick boxes and masks."""
+finished at once or after the walk, with and without brick boxes and masks. And the one-call
+area-light candidate (area_candidate) against the sample and target functions it stands for."""
 import ctypes as C
 import os
 import subprocess
@@ -120,3 +121,46 @@ def test_split_walk_finds_solid_cells(dh, split):  # noqa: F811
     hits, _, _ = _compare(dh, split, wa, O, D, rng.integers(0, 1 << 30, n), rng.choice([1, 8], n),
                           rng.choice([128, 30, 9], n))
     assert hits > 300
+
+
+def test_area_candidate_matches_sample_and_target(split):
+    """Wherever area_candidate answers, it gives the draws and the target value of
+    sample_area_light and phat bit for bit, and with a non-zero target the same point, weight
+    and face; it answers for nearly every ordinary candidate. Shading points far and near,
+    on face planes and inside the cube; huge and zero sizes, black and non-finite emission,
+    an RNG state of zero, points at infinity."""
+    rng = np.random.default_rng(17)
+    P = C.POINTER(C.c_float)
+    split.dh_area_candidate.argtypes = [P, C.c_uint32, C.c_uint32, P]
+    out = np.zeros((2, 7), np.float32)
+    answered = ordinary = lit = 0
+    for i in range(60000):
+        size = np.float32(rng.choice([1.0, 1.0, 8.0]))
+        c = np.floor(rng.uniform(0, 1000, 3)).astype(np.float32) + np.float32(0.5) * size
+        mode = i % 6
+        sp = rng.uniform(0, 1024, 3) if mode < 3 else c + rng.normal(0, 3 * size, 3)
+        if mode == 4:      # inside slabs, on face planes
+            sp = c + np.where(rng.random(3) < 0.5, rng.choice([-0.5, 0.5, 0.25], 3) * size, rng.normal(0, 9, 3))
+        em, brdf = rng.uniform(0, 30, 3), rng.uniform(0, 0.32, 3)
+        side, sign, seed = int(rng.integers(3)), float(rng.choice([-1.0, 1.0])), int(rng.integers(1, 2 ** 32))
+        if mode == 5:
+            k = i // 6 % 7
+            if k == 0: size = np.float32(rng.choice([0.0, 3.0, 5e5, 4e9]))   # noqa: E701
+            if k == 1: em = em * rng.choice([0.0, np.inf, np.nan, 1e30])     # noqa: E701
+            if k == 2: brdf = brdf * rng.choice([0.0, 1e-25, 1e25])          # noqa: E701
+            if k == 3: seed = 0                                              # noqa: E701
+            if k == 4: sp[int(rng.integers(3))] = rng.choice([np.inf, -np.inf, np.nan, 1e9])   # noqa: E701
+            if k == 5: sp = c.copy()                                         # noqa: E701
+        sp = sp.astype(np.float32)
+        spo = sp.copy()
+        spo[side] += np.float32(0.1) * np.float32(sign)
+        args = np.concatenate([c, [size], em, sp, spo, [sign], brdf]).astype(np.float32)
+        ok = split.dh_area_candidate(args.ctypes.data_as(P), side, seed, out.ctypes.data_as(P))
+        a, b = out.view(np.uint32)
+        if ok:
+            assert a[0] == b[0] and a[1] == b[1], (i, args, out)
+            assert out[0, 0] == 0.0 or (a[2:] == b[2:]).all(), (i, args, out)
+        answered += ok and mode < 3
+        ordinary += mode < 3
+        lit += bool(ok and out[0, 0] > 0)
+    assert answered > 0.999 * ordinary and lit > 10000
