@@ -58,21 +58,6 @@ __global__ void build_light_table_kernel(const uint4* __restrict__ raw, uint32_t
     emit[i] = make_float4((c.x * m) * INVPI, (c.y * m) * INVPI, (c.z * m) * INVPI, __uint_as_float(l.x));
 }
 
-// updateUberGrid (kernels.cl:498-513): 1 when any of the 4^3 grid cells is non-empty.
-__global__ void build_uber_kernel(const uint32_t* __restrict__ grid, uint8_t* uber) {
-    const int task = blockIdx.x * blockDim.x + threadIdx.x;
-    if (task >= 32 * 32 * 32) return;
-    const int x = task & 31, z = (task >> 5) & 31, y = task >> 10;
-    bool empty = true;
-    for (int a = 0; a < 4 && empty; a++)
-        for (int b = 0; b < 4 && empty; b++)
-            for (int c = 0; c < 4; c++) {
-                const int gx = x * 4 + a, gy = y * 4 + b, gz = z * 4 + c;
-                if (grid[gx + gz * 128 + gy * 16384]) { empty = false; break; }
-            }
-    uber[x + z * 32 + y * 1024] = empty ? 0 : 1;
-}
-
 // Per brick the boxes of its opaque voxels (type nibble 15) and of its non-zero voxels,
 // packed as World::bbox describes, and its opacity mask (World::bmask): one warp per brick,
 // 16 voxels a lane, min / max reductions over the warp, a ballot per mask word.
@@ -127,51 +112,69 @@ __global__ void commit_bricks_kernel(const uint32_t* __restrict__ list, const ui
     reinterpret_cast<uint4*>(bricks + (size_t)b * 512u)[threadIdx.x] = v;
 }
 
-// Per uber cell the box of its non-zero voxels (World::ubox0, null: not wanted): brick-less
-// non-zero grid cells count whole, bricks with their non-zero box (bbox0, built before);
-// and the cell's mask for shadow rays (World::ucell): the grid cells that can stop one (bbox,
-// null: every brick might).
-__global__ void build_uber_boxes_kernel(const uint32_t* __restrict__ grid, const uint32_t* __restrict__ bbox,
-                                        const uint32_t* __restrict__ bbox0, uint32_t* __restrict__ ubox0,
-                                        unsigned long long* __restrict__ ucell) {
-    const int task = blockIdx.x * blockDim.x + threadIdx.x;
-    if (task >= 32 * 32 * 32) return;
-    const int x = task & 31, z = (task >> 5) & 31, y = task >> 10;
-    uint32_t lo[3] = {31u, 31u, 31u}, hi[3] = {0u, 0u, 0u}, mask[2] = {0u, 0u};
-    bool any = false, occupied = false;
-    for (int b = 0; b < 64; b++) {
-        const uint32_t cx = b & 3, cz = (b >> 2) & 3, cy = b >> 4;
-        const uint32_t c = __ldg(grid + (x * 4 + cx) + (z * 4 + cz) * 128 + (y * 4 + cy) * 16384);
-        if (c == 0u) continue;
-        occupied = true;
-        const bool stops = (c & 1u) ? (!bbox || __ldg(bbox + (c >> 1)) != kNoOpaque) : (((c >> 1) & 0xf000u) >> 12) == 15u;
-        if (stops) mask[b >> 5] |= 1u << (b & 31);
-        uint32_t l[3] = {0u, 0u, 0u}, h[3] = {7u, 7u, 7u};
-        if (bbox0 && (c & 1u)) {
-            const uint32_t bb = __ldg(bbox0 + (c >> 1));
-            if (bb == kNoOpaque) continue;
-            for (int a = 0; a < 3; a++) { l[a] = (bb >> (3 * a)) & 7u; h[a] = (bb >> (9 + 3 * a)) & 7u; }
-        }
-        const uint32_t base[3] = {cx * 8u, cy * 8u, cz * 8u};
-        for (int a = 0; a < 3; a++) { lo[a] = min(lo[a], base[a] + l[a]); hi[a] = max(hi[a], base[a] + h[a]); }
-        any = true;
-    }
-    if (ubox0) {
-        uint32_t box = 0u;
-        for (int a = 0; a < 3; a++) box |= (lo[a] << (5 * a)) | (hi[a] << (15 + 5 * a));
-        ubox0[task] = any ? box : kNoOpaque;
-    }
-    if (occupied && !(mask[0] | mask[1])) mask[0] = 1u;
-    ucell[task] = mask[0] | ((unsigned long long)mask[1] << 32);
-}
-
-
-// World::gbox: every grid cell with its brick's opaque box
-__global__ void build_cell_boxes_kernel(const uint32_t* __restrict__ grid, const uint32_t* __restrict__ bbox,
-                                        uint2* __restrict__ gbox) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;   // 128^3 threads
+// The tables that follow from the grid and the brick boxes, two warps per uber cell, a lane
+// per grid cell:
+//   uber    updateUberGrid (kernels.cl:498-513): 1 when any of the 4^3 grid cells is non-empty
+//   ucell   World::ucell; ucell0 World::ucell0 (with the box: brick-less non-zero cells count
+//           whole, bricks with their non-zero box)
+//   gbox, gbox0   World::gbox, gbox0, unless null
+// bbox, bbox0 null: no brick boxes (every brick may hold anything); nbricks, err: a grid cell
+// that points past nbricks bricks raises flag 16 (err null: not checked). With one thread
+// per uber cell reading its 64 cells in turn this took 59 us for 107,384 bricks (and the
+// uber grid 12, the cell boxes 9, each a launch); 13 us this way.
+struct CellTables {
+    uint8_t* uber;
+    unsigned long long* ucell;
+    uint4* ucell0;
+    uint2 *gbox, *gbox0;
+};
+__global__ void __launch_bounds__(256) build_cells_kernel(const uint32_t* __restrict__ grid, const uint32_t* __restrict__ bbox,
+                                                          const uint32_t* __restrict__ bbox0, const CellTables out,
+                                                          uint32_t nbricks, uint32_t* err) {
+    __shared__ uint32_t s_mask[8], s_mask0[8], s_lo[8][3], s_hi[8][3];
+    __shared__ bool s_occ[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t u = blockIdx.x * 4u + (uint32_t)(warp >> 1);            // x + z*32 + y*1024
+    const uint32_t b = (uint32_t)(warp & 1) * 32u + (uint32_t)lane;        // x + z*4 + y*16 inside it
+    const uint32_t cx = b & 3u, cz = (b >> 2) & 3u, cy = b >> 4;
+    const uint32_t i = ((u & 31u) * 4u + cx) + (((u >> 5) & 31u) * 4u + cz) * 128u + ((u >> 10) * 4u + cy) * 16384u;
     const uint32_t c = __ldg(grid + i);
-    gbox[i] = make_uint2(c, (c & 1u) ? __ldg(bbox + (c >> 1)) : 0u);
+    const bool brick = c & 1u;
+    if (err && brick && (c >> 1) >= nbricks) atomicOr(err, 16u);
+    const uint32_t box = brick && bbox ? __ldg(bbox + (c >> 1)) : 0u, box0 = brick && bbox0 ? __ldg(bbox0 + (c >> 1)) : 0u;
+    if (out.gbox) out.gbox[i] = make_uint2(c, box);
+    if (out.gbox0) out.gbox0[i] = make_uint2(c, box0);
+    const bool stops = brick ? box != kNoOpaque : (((c >> 1) & 0xf000u) >> 12) == 15u;
+    const bool stops0 = c != 0u && !(brick && box0 == kNoOpaque);
+    const uint32_t m = __ballot_sync(0xffffffffu, stops), m0 = __ballot_sync(0xffffffffu, stops0);
+    const bool occ = __any_sync(0xffffffffu, c != 0u);
+    const uint32_t at[3] = {cx * 8u, cy * 8u, cz * 8u};
+    uint32_t lo[3], hi[3];
+    for (int a = 0; a < 3; a++) {
+        const uint32_t l = brick && bbox0 ? (box0 >> (3 * a)) & 7u : 0u, h = brick && bbox0 ? (box0 >> (9 + 3 * a)) & 7u : 7u;
+        lo[a] = __reduce_min_sync(0xffffffffu, stops0 ? at[a] + l : 31u);
+        hi[a] = __reduce_max_sync(0xffffffffu, stops0 ? at[a] + h : 0u);
+    }
+    if (lane == 0) {
+        s_mask[warp] = m;
+        s_mask0[warp] = m0;
+        s_occ[warp] = occ;
+        for (int a = 0; a < 3; a++) { s_lo[warp][a] = lo[a]; s_hi[warp][a] = hi[a]; }
+    }
+    __syncthreads();
+    if (lane == 0 && !(warp & 1)) {
+        const bool any = s_occ[warp] || s_occ[warp + 1];
+        uint32_t k[2] = {s_mask[warp], s_mask[warp + 1]}, k0[2] = {s_mask0[warp], s_mask0[warp + 1]};
+        uint32_t ubox = 0u;
+        for (int a = 0; a < 3; a++)
+            ubox |= (min(s_lo[warp][a], s_lo[warp + 1][a]) << (5 * a)) | (max(s_hi[warp][a], s_hi[warp + 1][a]) << (15 + 5 * a));
+        if (!(k0[0] | k0[1])) ubox = kNoOpaque;
+        if (any && !(k[0] | k[1])) k[0] = 1u;
+        if (any && !(k0[0] | k0[1])) k0[0] = 1u;
+        out.uber[u] = any ? 1 : 0;
+        out.ucell[u] = k[0] | ((unsigned long long)k[1] << 32);
+        out.ucell0[u] = make_uint4(k0[0], k0[1], ubox, 0u);
+    }
 }
 
 // ---- work distribution --------------------------------------------------------------------
@@ -248,8 +251,11 @@ __device__ __forceinline__ bool next_tile(const BatchDev& bd, uint32_t* ctr, uin
     return s_tile < bd.totalTiles;
 }
 
-// view of a batch tile and the pixel of this thread in it
-template <int VARIANT>
+// View of a batch tile and the pixel of this thread in it. RAYS: a warp takes 8 x 4 pixels of
+// the tile where its sides allow (else, and for stages that read and write planes, rows
+// in order): the primary rays of a compact block cross the same cells longer than those of
+// 16 x 2 pixels (1080p, 65,536 emitters: 393 us against 413).
+template <int VARIANT, bool RAYS = false>
 __device__ __forceinline__ const ViewDev* tile_pixel(const BatchDev& bd, uint32_t tile, int* x, int* y) {
     uint32_t v = 0;
     if (VARIANT == 2)
@@ -257,8 +263,14 @@ __device__ __forceinline__ const ViewDev* tile_pixel(const BatchDev& bd, uint32_
     const ViewDev* V = view_of<VARIANT>(bd, v);
     const uint32_t lt = tile - V->tileBase;
     const uint32_t tx = lt % V->tilesX, ty = lt / V->tilesX;
-    *x = (int)(tx * (uint32_t)bd.tx + threadIdx.x % (uint32_t)bd.tx);
-    *y = (int)(ty * (uint32_t)bd.ty + threadIdx.x / (uint32_t)bd.tx);
+    uint32_t ix = threadIdx.x % (uint32_t)bd.tx, iy = threadIdx.x / (uint32_t)bd.tx;
+    if (RAYS && (((uint32_t)bd.tx & 7u) | ((uint32_t)bd.ty & 3u)) == 0u) {
+        const uint32_t warp = threadIdx.x >> 5, across = (uint32_t)bd.tx >> 3;
+        ix = (warp % across) * 8u + (threadIdx.x & 7u);
+        iy = (warp / across) * 4u + ((threadIdx.x >> 3) & 3u);
+    }
+    *x = (int)(tx * (uint32_t)bd.tx + ix);
+    *y = (int)(ty * (uint32_t)bd.ty + iy);
     return V;
 }
 
@@ -269,7 +281,7 @@ __device__ __forceinline__ void albedo_px(const World& w, const Frame& k, uint2*
     const float3 D = camera_ray(k, x, y);
     uint32_t side = 0;
     float dist = 0.0f;
-    uint32_t voxel = trace<0>(w, k.E.x, k.E.y, k.E.z, D.x, D.y, D.z, 999999, 0u, 0u, &dist, &side);
+    uint32_t voxel = trace_primary(w, k.E, D, &dist, &side);
     float alpha = alphaf(voxel);
     float3 outc = mul(to_rgb(voxel), alpha);
     float total = 0.0f;
@@ -298,12 +310,16 @@ __device__ __forceinline__ void albedo_px(const World& w, const Frame& k, uint2*
     seeds[i] = seed;
 }
 
+// Bound by instruction issue; 4 blocks of 256 threads a SM (64 registers) measured faster than
+// 3 (1080p: 413 us against 446) and 5 (455). trace_first's cell masks and packed cells, these
+// blocks and compact warps: 1080p, 65,536 emitters 544 -> 393 us, 3840 x 2160 with 1,048,576
+// emitters 3,099 -> 2,103 us.
 template <int VARIANT>
-__global__ void __launch_bounds__(kMaxTileThreads) albedo_kernel(const __grid_constant__ BatchDev bd) {
+__global__ void __launch_bounds__(kMaxTileThreads, 4) albedo_kernel(const __grid_constant__ BatchDev bd) {
     uint32_t tile, round = 0;
     while (next_tile(bd, bd.counters + kCtrAlbedo, &tile, round)) {
         int x, y;
-        const ViewDev* V = tile_pixel<VARIANT>(bd, tile, &x, &y);
+        const ViewDev* V = tile_pixel<VARIANT, true>(bd, tile, &x, &y);
         const Frame& k = V->k;
         if (x < k.W && y < k.H) {
             const World w = V->w;
@@ -343,7 +359,7 @@ __device__ __forceinline__ float4 path_trace_px(const World& w, const Frame& k, 
     const float3 D = camera_ray(k, x, y);
     float dist = 0.0f;
     uint32_t side = 0;
-    const uint32_t voxel = trace<0>(w, k.E.x, k.E.y, k.E.z, D.x, D.y, D.z, 999999, 0u, 0u, &dist, &side);
+    const uint32_t voxel = trace_primary(w, k.E, D, &dist, &side);
     if (voxel == 0u) return make_float4(0.0f, 0.0f, 0.0f, 1e20f);
     const float INVPI = 0.31830988618379067153777f;
     const float3 rgb = to_rgb(voxel);
@@ -360,8 +376,8 @@ __device__ __forceinline__ float4 path_trace_px(const World& w, const Frame& k, 
     const float NdotL = fmaxf(0.0f, (N.x * R.x + N.y * R.y) + N.z * R.z);
     float dist2 = 0.0f;
     uint32_t side2 = 0;
-    const uint32_t voxel2 = trace<0>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z, 128, 0u, 0u,
-                                     &dist2, &side2);
+    const uint32_t voxel2 = trace_first<true, true>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z,
+                                                    128, &dist2, &side2);
     const float3 sampleL = mul(mul(to_rgb(voxel2), (float)((voxel2 & 0xff0000u) >> 16)), INVPI);
     const float TWOPI = 6.28318530717958647692528f;
     return make_float4(((sampleL.x * TWOPI) * NdotL) * brdf.x + contribution.x,
@@ -369,11 +385,11 @@ __device__ __forceinline__ float4 path_trace_px(const World& w, const Frame& k, 
                        ((sampleL.z * TWOPI) * NdotL) * brdf.z + contribution.z, dist);
 }
 
-__global__ void __launch_bounds__(kMaxTileThreads) path_trace_kernel(const __grid_constant__ BatchDev bd) {
+__global__ void __launch_bounds__(kMaxTileThreads, 4) path_trace_kernel(const __grid_constant__ BatchDev bd) {
     uint32_t tile, round = 0;
     while (next_tile(bd, bd.counters + kCtrAlbedo, &tile, round)) {
         int x, y;
-        const ViewDev* V = tile_pixel<0>(bd, tile, &x, &y);
+        const ViewDev* V = tile_pixel<0, true>(bd, tile, &x, &y);
         const Frame& k = V->k;
         if (x < k.W && y < k.H) V->b.frame[(size_t)y * k.W + x] = path_trace_px(V->w, k, x, y);
     }
@@ -1274,10 +1290,6 @@ void launch_build_light_table(const uint4* raw, uint32_t n, float4* geom, float4
     dev::build_light_table_kernel<<<(n + 255) / 256, 256, 0, s>>>(raw, n, geom, emit);
 }
 
-void launch_build_uber(const uint32_t* grid, uint8_t* uber, cudaStream_t s) {
-    dev::build_uber_kernel<<<(32 * 32 * 32 + 255) / 256, 256, 0, s>>>(grid, uber);
-}
-
 void launch_build_brick_boxes(const uint32_t* bricks, const uint32_t* list, uint32_t n, uint32_t* bbox, uint32_t* bbox0,
                               uint32_t* bmask, cudaStream_t s) {
     const size_t threads = (size_t)n * 32u;
@@ -1289,13 +1301,11 @@ void launch_commit_bricks(const uint32_t* list, const uint32_t* voxels, uint32_t
     if (n) dev::commit_bricks_kernel<<<n, 128, 0, s>>>(list, voxels, bricks);
 }
 
-void launch_build_uber_boxes(const uint32_t* grid, const uint32_t* bbox, const uint32_t* bbox0, uint32_t* ubox0,
-                             unsigned long long* ucell, cudaStream_t s) {
-    dev::build_uber_boxes_kernel<<<(32 * 32 * 32 + 63) / 64, 64, 0, s>>>(grid, bbox, bbox0, ubox0, ucell);
-}
-
-void launch_build_cell_boxes(const uint32_t* grid, const uint32_t* bbox, uint2* gbox, cudaStream_t s) {
-    dev::build_cell_boxes_kernel<<<128 * 128 * 128 / 256, 256, 0, s>>>(grid, bbox, gbox);
+void launch_build_cells(const uint32_t* grid, const uint32_t* bbox, const uint32_t* bbox0, uint8_t* uber,
+                        unsigned long long* ucell, uint4* ucell0, uint2* gbox, uint2* gbox0, uint32_t nbricks, uint32_t* err,
+                        cudaStream_t s) {
+    const dev::CellTables out{uber, ucell, ucell0, gbox, gbox0};
+    dev::build_cells_kernel<<<32 * 32 * 32 / 4, 256, 0, s>>>(grid, bbox, bbox0, out, nbricks, err);
 }
 
 void launch_path_trace(const BatchDev& bd, cudaStream_t s) {

@@ -46,7 +46,7 @@ static_assert(kScratchBytes == VXR_NOALLOC_SCRATCH_BYTES, "scratch size must mat
 static_assert(kOffSeed % 256 == 0 && kOffCA % 256 == 0 && kOffUber % 256 == 0 && kOffGeom % 256 == 0 &&
                   kOffHits % 256 == 0 && kOffQA % 256 == 0 && kOffErr % 256 == 0,
               "scratch regions must stay 256-byte aligned");
-static_assert(16 * kMaxLights >= 8 * 32 * 32 * 32, "the uber cells' masks must fit the region of the widened lights");
+static_assert(16 * kMaxLights >= (16 + 8) * 32 * 32 * 32, "the uber cells' masks must fit the region of the widened lights");
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -78,14 +78,6 @@ int scratch_for_current_device(unsigned char** out) {
 __global__ void widen_lights_kernel(const vxr_light* __restrict__ in, uint32_t n, uint4* out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = make_uint4(in[i].position, in[i].voxel, in[i].size, 0u);
-}
-
-// every brick cell of the grid must index inside the caller's brick array
-__global__ void check_grid_kernel(const uint32_t* __restrict__ grid, uint32_t nbricks, uint32_t* err) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 128u * 128u * 128u) return;
-    const uint32_t c = grid[i];
-    if ((c & 1u) && (c >> 1) >= nbricks) atomicOr(err, 16u);
 }
 
 }  // namespace
@@ -120,15 +112,8 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     uint32_t* err = (uint32_t*)(s + kOffErr);
     CUN(cudaMemsetAsync(err, 0, sizeof(uint32_t), st), "clear error word");
 
-    // validate the grid before any traversal reads the bricks through it
-    check_grid_kernel<<<(128 * 128 * 128 + 255) / 256, 256, 0, st>>>(grid, nbricks, err);
-    CUN(cudaGetLastError(), "grid check");
-    uint32_t herr = 0;
-    CUN(cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "read error word");
-    CUN(cudaStreamSynchronize(st), "grid check");
-    if (herr & 16u) return vxr::set_error(VXR_E_INVALID, "vxr_render_frame_noalloc: grid references a brick >= nbricks");
-
-    // derive the uber grid and the light table in scratch
+    // derive the light table and the uber cells' tables in scratch; the latter's kernel also
+    // validates the grid, before any traversal reads the bricks through it
     uint4* raw = (uint4*)(s + kOffRaw);
     float4* geom = (float4*)(s + kOffGeom);
     float4* emit = (float4*)(s + kOffEmit);
@@ -136,12 +121,16 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
         widen_lights_kernel<<<(nlights + 255) / 256, 256, 0, st>>>(lights, nlights, raw);
         vxr::launch_build_light_table(raw, nlights, geom, emit, st);
     }
-    vxr::launch_build_uber(grid, s + kOffUber, st);
     // the uber cells' masks take the place of the widened lights, which only the light
     // table's kernel reads
-    unsigned long long* ucell = (unsigned long long*)raw;
-    vxr::launch_build_uber_boxes(grid, nullptr, nullptr, nullptr, ucell, st);
+    uint4* ucell0 = raw;
+    unsigned long long* ucell = (unsigned long long*)(ucell0 + 32 * 32 * 32);
+    vxr::launch_build_cells(grid, nullptr, nullptr, s + kOffUber, ucell, ucell0, nullptr, nullptr, nbricks, err, st);
     CUN(cudaGetLastError(), "world kernels");
+    uint32_t herr = 0;
+    CUN(cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "read error word");
+    CUN(cudaStreamSynchronize(st), "grid check");
+    if (herr & 16u) return vxr::set_error(VXR_E_INVALID, "vxr_render_frame_noalloc: grid references a brick >= nbricks");
 
     vxr::dev::World w;
     w.grid = grid;
@@ -151,6 +140,7 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     w.bbox0 = nullptr;
     w.ubox0 = nullptr;
     w.ucell = ucell;
+    w.ucell0 = ucell0;
     w.lgeom = geom;
     w.lemit = emit;
     w.nlights = nlights;

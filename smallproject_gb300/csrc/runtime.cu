@@ -36,7 +36,7 @@ void release_device_world(World& w) {
     cudaFree(d->bricks);
     cudaFree(d->bbox);
     cudaFree(d->bmask);
-    cudaFree(d->ubox0);
+    cudaFree(d->ucell0);
     cudaFree(d->ucell);
     cudaFree(d->gbox);
     cudaFree(d->stageDev);
@@ -73,9 +73,10 @@ static int upload(World& w) {
     d.device = dev;
     if (!d.grid) CU(cudaMalloc(&d.grid, kGridSize * sizeof(uint32_t)), "cudaMalloc(grid)");
     if (!d.uber) CU(cudaMalloc(&d.uber, 32 * 32 * 32), "cudaMalloc(uber)");
-    if (!d.ubox0) CU(cudaMalloc(&d.ubox0, 32 * 32 * 32 * sizeof(uint32_t)), "cudaMalloc(uber boxes)");
+    if (!d.ucell0) CU(cudaMalloc(&d.ucell0, 32 * 32 * 32 * sizeof(uint4)), "cudaMalloc(uber boxes)");
     if (!d.ucell) CU(cudaMalloc(&d.ucell, 32 * 32 * 32 * sizeof(unsigned long long)), "cudaMalloc(uber cells)");
-    if (!d.gbox) CU(cudaMalloc(&d.gbox, kGridSize * sizeof(uint2)), "cudaMalloc(cell boxes)");
+    if (!d.gbox) CU(cudaMalloc(&d.gbox, 2 * (size_t)kGridSize * sizeof(uint2)), "cudaMalloc(cell boxes)");
+    d.gbox0 = d.gbox + kGridSize;
     uint32_t sent = 0;
     if (full) {
         if (w.brickHigh > d.cap || !d.bricks) {
@@ -150,12 +151,9 @@ static int upload(World& w) {
                 y = e;
             }
         }
-        launch_build_uber(d.grid, d.uber, 0);
     }
-    if (full || w.gridDirty || sent) {
-        launch_build_uber_boxes(d.grid, d.bbox, d.bbox0, d.ubox0, d.ucell, 0);
-        launch_build_cell_boxes(d.grid, d.bbox, d.gbox, 0);
-    }
+    if (full || w.gridDirty || sent)
+        launch_build_cells(d.grid, d.bbox, d.bbox0, d.uber, d.ucell, d.ucell0, d.gbox, d.gbox0, 0, nullptr, 0);
     if (full || d.lightVersion != w.lightVersion || d.lightMoveVersion != w.lightMoveVersion) {
         const uint32_t nl = (uint32_t)w.lights.size();
         const size_t need = std::max<uint32_t>(nl, 1u);
@@ -217,10 +215,12 @@ vxr::dev::World dev_world(vxr_view* v) {
     w.bricks = d.bricks;
     w.bbox = d.bbox;
     w.bbox0 = d.bbox0;
-    w.ubox0 = d.ubox0;
+    w.ubox0 = nullptr;
+    w.ucell0 = d.ucell0;
     w.ucell = d.ucell;
     w.bmask = d.bmask;
     w.gbox = d.gbox;
+    w.gbox0 = d.gbox0;
     w.lgeom = d.lgeom;
     w.lemit = d.lemit;
     w.nlights = d.nl;
@@ -474,8 +474,8 @@ int vxr_world_pending(const vxr_world* w, uint32_t* dirty_bricks, int* grid_chan
 int vxr_world_device_bytes(const vxr_world* w, uint64_t* bytes) {
     VXR_CHECK_ARG(w && bytes, "vxr_world_device_bytes: null argument");
     const vxr::DeviceWorld* d = w->w.dev;
-    // grid and its boxes, uber grid, its boxes and masks, bricks, their boxes and masks, light tables
-    *bytes = d ? (uint64_t)(vxr::kGridSize * 12 + 32768 + 32768 * 4 + 32768 * 8 + (uint64_t)d->cap * (vxr::kBrick * 4 + 8 + 64) +
+    // grid and its two box tables, uber grid and its masks, bricks, their boxes and masks, light tables
+    *bytes = d ? (uint64_t)(vxr::kGridSize * 20 + 32768 + 32768 * 16 + 32768 * 8 + (uint64_t)d->cap * (vxr::kBrick * 4 + 8 + 64) +
                             (uint64_t)d->stageCap * (vxr::kBrick + 1) * 4 + d->lcap * 48)
                : 0;
     return VXR_OK;

@@ -1,6 +1,6 @@
 // devhost_split.cpp - the split shadow DDA (GridWalk, grid_task, brick_task in device.cuh)
 // run on the host, one ray at a time, tasks in visiting order, as the tracer's queues keep
-// them; and the one-call area-light candidate. Test infrastructure only.
+// them; the first-voxel trace over cell masks; and the one-call area-light candidate. Test infrastructure only.
 #include "devhost.cpp"
 
 extern "C" {
@@ -68,6 +68,19 @@ int dh_shadow_split(const uint32_t* grid, const uint32_t* bricks, const uint32_t
     const uint32_t vz = f2u(hz - (s2 == 2 ? ns * 0.1f : 0.0f));
     const uint32_t ey = pos / (1024u * 1024u), ez = (pos / 1024u) % 1024u, ex = pos % 1024u;
     return ex <= vx && ex + size > vx && ey <= vy && ey + size > vy && ez <= vz && ez + size > vz;
+}
+
+// trace_first with a budget, or a primary ray (boxes: gbox0 given)
+uint32_t dh_trace_first(const uint32_t* grid, const uint8_t* uber, const uint32_t* bricks, const uint32_t* ucell0, const uint32_t* gbox0,
+                        const float* O, const float* D, int budget, int steps, float* dist, uint32_t* side) {
+    World w = make_world(grid, uber, bricks);
+    w.ucell0 = reinterpret_cast<const uint4*>(ucell0);
+    w.gbox0 = reinterpret_cast<const uint2*>(gbox0);
+    *dist = 0.0f;
+    *side = 0;
+    if (!budget) return trace_primary(w, f3(O[0], O[1], O[2]), f3(D[0], D[1], D[2]), dist, side);
+    const auto f = gbox0 ? trace_first<true, true> : trace_first<false, true>;
+    return f(w, O[0], O[1], O[2], D[0], D[1], D[2], steps, dist, side);
 }
 
 // An area-light candidate: one call (area_candidate) and the two functions it stands for.

@@ -1,6 +1,7 @@
 """The split shadow DDA (GridWalk and its tasks, device.cuh) compiled for the CPU, against the
 resumable walker: the same status, distance bits, side and visibility for every ray, tasks
-finished at once or after the walk, with and without brick boxes and masks. And the one-call
+finished at once or after the walk, with and without brick boxes and masks. The first-voxel trace over cell masks (trace_first)
+against the three-level DDA it stands for. And the one-call
 area-light candidate (area_candidate) against the sample and target functions it stands for."""
 import ctypes as C
 import os
@@ -11,7 +12,8 @@ import pytest
 
 from conftest import ROOT
 from oracle import binding as ob
-from test_device_code_host import _candidate_shadow_rays, _f3, _rays, _surface_rays, brick_boxes, dh  # noqa: F401
+from test_device_code_host import (_candidate_shadow_rays, _f3, _rays, _surface_rays, brick_boxes, dh,  # noqa: F401
+                                   uber_boxes0)
 
 NATIVE = os.path.join(ROOT, "tests", "native")
 
@@ -44,6 +46,26 @@ def uber_cells(grid, bricks, boxes):
     occupied = (g != 0).reshape(32, 4, 32, 4, 32, 4).any(axis=(1, 3, 5))
     out[..., 0] |= (occupied & ~out.any(axis=-1)).astype(np.uint32)
     return np.ascontiguousarray(out.reshape(-1, 2))
+
+
+def uber_cells0(grid, bricks, boxed):
+    """World::ucell0 and gbox0 as the GPU builds them (build_cells_kernel); boxed False: every
+    brick counts as one that can stop a ray, and there is no gbox0."""
+    g = grid.reshape(128, 128, 128)
+    box = brick_boxes(bricks, nonzero=True)
+    brick = (g & 1) == 1
+    stops = g != 0
+    if boxed:
+        stops[brick] = box[g[brick] >> 1] != 0xFFFFFFFF
+    out = np.zeros((32, 32, 32, 4), np.uint32)
+    for b in range(64):
+        s = stops[b >> 4::4, (b >> 2) & 3::4, b & 3::4].astype(np.uint32)
+        out[..., b >> 5] |= s << np.uint32(b & 31)
+    occupied = (g != 0).reshape(32, 4, 32, 4, 32, 4).any(axis=(1, 3, 5))
+    out[..., 2] = uber_boxes0(grid, bricks).reshape(32, 32, 32)
+    out[..., 0] |= (occupied & ~out[..., :2].any(axis=-1)).astype(np.uint32)
+    gbox = np.stack([grid, np.where(grid & 1, box[np.where(grid & 1, grid >> 1, 0)], 0).astype(np.uint32)], 1) if boxed else None
+    return np.ascontiguousarray(out.reshape(-1, 4)), gbox
 
 
 def brick_masks(bricks):
@@ -121,6 +143,59 @@ def test_split_walk_finds_solid_cells(dh, split):  # noqa: F811
     hits, _, _ = _compare(dh, split, wa, O, D, rng.integers(0, 1 << 30, n), rng.choice([1, 8], n),
                           rng.choice([128, 30, 9], n))
     assert hits > 300
+
+
+def _compare_first(dh, split, wa, O, D, stepss):  # noqa: F811
+    P = lambda a: a.ctypes.data if a is not None else None  # noqa: E731
+    split.dh_trace_first.restype = C.c_uint32
+    split.dh_trace_first.argtypes = [C.c_void_p] * 5 + [C.POINTER(C.c_float)] * 2 + [C.c_int, C.c_int, C.POINTER(C.c_float),
+                                                                                     C.POINTER(C.c_uint32)]
+    hits = 0
+    for boxed in (True, False):
+        uc, gb = uber_cells0(wa.grid, wa.bricks, boxed)
+        for i in range(len(O)):
+            o, d, steps = _f3(O[i]), _f3(D[i]), int(stepss[i])
+            da, sa, db, sb = C.c_float(0), C.c_uint32(0), C.c_float(0), C.c_uint32(0)
+            a = dh.dh_trace(0, P(wa.grid), P(wa.uber), P(wa.bricks), o, d, steps, 0, 0, C.byref(da), C.byref(sa))
+            b = split.dh_trace_first(P(wa.grid), P(wa.uber), P(wa.bricks), P(uc), P(gb), o, d, int(steps < 999999), steps, C.byref(db),
+                                     C.byref(sb))
+            assert (a, sa.value) == (b, sb.value) and \
+                np.float32(da.value).view(np.uint32) == np.float32(db.value).view(np.uint32), (i, O[i], D[i], steps)
+            hits += a != 0
+    return hits
+
+
+def test_trace_first_matches_trace(dh, split, world0_arrays):  # noqa: F811
+    """Terrain with emitters: rays from inside and outside the map, leaving the surface, axis
+    aligned and of numbers that are not finite, endless and with budgets down to one step."""
+    wa = world0_arrays
+    o1, d1, rng = _rays(2500, 91)
+    o2, d2, _ = _surface_rays(wa, 1500, 92)
+    n, i = np.nan, np.inf
+    d3 = np.float32([[0, -1, 0], [n, n, n], [i, 0, 0], [n, 0, -1], [i, n, n], [0, i, 0], [0.6, n, 0.8], [0, 0, 0]])
+    o3 = np.tile(np.float32([[128.5, 200.5, 128.5]]), (len(d3), 1))
+    o4, d4 = np.float32([[n, n, n], [i, 5, 5], [-i, i, n], [5, 5, -1e35]]), np.tile(np.float32([[0.6, 0, 0.8]]), (4, 1))
+    O, D = np.concatenate([o1, o2, o3, o4]), np.concatenate([d1, d2, d3, d4])
+    steps = rng.choice([999999, 999999, 128, 128, 9, 5, 4, 1], len(O))
+    steps[-12:] = 999999
+    assert _compare_first(dh, split, wa, O, D, steps) > 1500
+
+
+def test_trace_first_matches_trace_on_solid_cells(dh, split):  # noqa: F811
+    """Brick-less cells, bricks without a non-zero voxel, single voxels in the air."""
+    import smallproject_gb300 as vx
+    w = vx.World()
+    rng = np.random.default_rng(8)
+    for b in rng.integers(0, 16, (160, 3)):
+        w.add_brick(int(b[0]), int(b[1]), int(b[2]), 0xF123 if rng.random() < 0.5 else 0x8123)
+    for k, b in enumerate(rng.integers(0, 128, (400, 3))):
+        w.set(int(b[0]), int(b[1]), int(b[2]), 0xFFFF)
+        if k % 3 == 0:
+            w.set(int(b[0]), int(b[1]), int(b[2]), 0)
+    g, bricks, lights = w.arrays()
+    wa = ob.WorldArrays(g, bricks, lights)
+    O, D, rng = _rays(2500, 16, lo=-40.0, hi=170.0, inside=(0.0, 128.0))
+    assert _compare_first(dh, split, wa, O, D, rng.choice([999999, 128, 30, 9], len(O))) > 800
 
 
 def test_area_candidate_matches_sample_and_target(split):
