@@ -189,6 +189,7 @@ int vxr_batch_create(vxr_view* const* views, uint32_t n, uint32_t tile_x, uint32
         bd.totalTiles = (uint32_t)tl;
         vxr::apply_tuning(bd, tu);
         bd.fuse = 1;
+        bd.lists = 1;
         dalloc((void**)&bd.hits, px * sizeof(uint32_t));
         dalloc((void**)&bd.qA, px * sizeof(float4));
         dalloc((void**)&bd.qB, px * sizeof(float4));

@@ -275,7 +275,7 @@ __device__ __forceinline__ const ViewDev* tile_pixel(const BatchDev& bd, uint32_
 }
 
 // ---- stage 1: primary rays / G-buffer (renderAlbedo, ris.cl:295-389) --------------------
-__device__ __forceinline__ void albedo_px(const World& w, const Frame& k, uint2* __restrict__ vd, uint32_t* __restrict__ seeds,
+__device__ __forceinline__ bool albedo_px(const World& w, const Frame& k, uint2* __restrict__ vd, uint32_t* __restrict__ seeds,
                                           int x, int y) {
     const uint32_t seed = wang_hash((uint32_t)x * 171u + (uint32_t)y * 1773u + k.R0);
     const float3 D = camera_ray(k, x, y);
@@ -308,23 +308,42 @@ __device__ __forceinline__ void albedo_px(const World& w, const Frame& k, uint2*
     const size_t i = (size_t)y * k.W + x;
     vd[i] = make_uint2(enc | (side << 24), __float_as_uint(total));
     seeds[i] = seed;
+    return (enc & 0x00FFFFFFu) != 0u;
+}
+
+// Where pixel i of the view (number v of its batch) goes after its primary ray: a hit pixel to
+// the hit list, the others get the empty reservoir (ris.cl:34,123). Every thread of a block
+// calls it together.
+__device__ __forceinline__ void list_pixel(const BatchDev& bd, const ViewDev* V, uint32_t v, uint32_t i, bool in, bool hit) {
+    const uint32_t slot = block_append(bd.counters + kCtrHits, hit);
+    if (hit) {
+        bd.hits[slot] = (v << 27) | i;
+    } else if (in) {
+        V->b.cA[i] = make_uint4(0u, 6u << 29, 0u, 0u);
+        V->b.cB[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
 }
 
 // Bound by instruction issue; 4 blocks of 256 threads a SM (64 registers) measured faster than
 // 3 (1080p: 413 us against 446) and 5 (455). trace_first's cell masks and packed cells, these
 // blocks and compact warps: 1080p, 65,536 emitters 544 -> 393 us, 3840 x 2160 with 1,048,576
 // emitters 3,099 -> 2,103 us.
-template <int VARIANT>
+// LISTS: the kernel also fills the hit list, in tile order (compact_hits_kernel reads the
+// G-buffer back for it: 333 x 187 271 -> 267 us a frame; at 1080p no difference).
+template <int VARIANT, bool LISTS>
 __global__ void __launch_bounds__(kMaxTileThreads, 4) albedo_kernel(const __grid_constant__ BatchDev bd) {
     uint32_t tile, round = 0;
     while (next_tile(bd, bd.counters + kCtrAlbedo, &tile, round)) {
         int x, y;
         const ViewDev* V = tile_pixel<VARIANT, true>(bd, tile, &x, &y);
         const Frame& k = V->k;
-        if (x < k.W && y < k.H) {
+        const bool in = x < k.W && y < k.H;
+        bool hit = false;
+        if (in) {
             const World w = V->w;
-            albedo_px(w, k, V->b.vd[V->cur], V->b.seed, x, y);
+            hit = albedo_px(w, k, V->b.vd[V->cur], V->b.seed, x, y);
         }
+        if (LISTS) list_pixel(bd, V, VARIANT < 2 ? 0u : (uint32_t)(V - bd.views), (uint32_t)y * (uint32_t)k.W + (uint32_t)x, in, hit);
     }
 }
 
@@ -395,27 +414,18 @@ __global__ void __launch_bounds__(kMaxTileThreads, 4) path_trace_kernel(const __
     }
 }
 
-// Hit list of the frame over every view (blockIdx.y = view); pixels without a hit get
-// the empty reservoir (ris.cl:34,123).
+// Hit list of the frame over every view (blockIdx.y = view), for frames run stage by stage
+// (whole frames fill it in the primary rays' kernel).
 template <int VARIANT>
 __global__ void __launch_bounds__(256) compact_hits_kernel(const __grid_constant__ BatchDev bd) {
     const ViewDev* V = view_of<VARIANT>(bd, blockIdx.y);
     const uint32_t n = (uint32_t)V->k.W * (uint32_t)V->k.H;
     const uint2* vd = V->b.vd[V->cur];
-    uint4* cA = V->b.cA;
-    float4* cB = V->b.cB;
-    // every thread of a block runs the same iterations (block_append needs all of them)
+    // every thread of a block runs the same iterations (list_pixel needs all of them)
     for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
         const uint32_t i = i0 + threadIdx.x;
         const bool in = i < n;
-        const bool hit = in && (vd[i].x & 0x00FFFFFFu) != 0u;
-        const uint32_t slot = block_append(bd.counters + kCtrHits, hit);
-        if (hit) {
-            bd.hits[slot] = (blockIdx.y << 27) | i;
-        } else if (in) {
-            cA[i] = make_uint4(0u, 6u << 29, 0u, 0u);
-            cB[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
+        list_pixel(bd, V, blockIdx.y, i, in, in && (vd[i].x & 0x00FFFFFFu) != 0u);
     }
 }
 
@@ -904,10 +914,38 @@ __global__ void __launch_bounds__(128) temporal_kernel(const __grid_constant__ B
     }
 }
 
+// 4a: the shadow-ray request of a hit pixel whose reservoir has W > 0 and M > 0; false without
+__device__ __forceinline__ bool shade_ray(const ViewDev* V, uint32_t e, int x, int y, uint2 g, uint32_t li, uint32_t M,
+                                          float sumW, float pHat, float3 pos, float4* ra, float4* rb) {
+    const Frame& k = V->k;
+    const float W = sumW / fmaxf(1e-5f, pHat * (float)M);
+    if (!(W > 0.0f && M > 0u)) return false;
+    const uint32_t side = g.x >> 24;
+    const float dist = __uint_as_float(g.y);
+    const float3 D = camera_ray(k, x, y);
+    const float nsign = side_sign(side, D);
+    const float3 sp = f3(D.x * dist + k.E.x, D.y * dist + k.E.y, D.z * dist + k.E.z);
+    const float3 spo = f3(sp.x + (side == 0 ? 0.1f * nsign : 0.0f), sp.y + (side == 1 ? 0.1f * nsign : 0.0f),
+                          sp.z + (side == 2 ? 0.1f * nsign : 0.0f));
+    if (li >= k.nlights) { raise_error(V->b.err, 8u); li = 0; }
+    const float3 L = normalize3(sub(pos, spo));
+    *ra = make_float4(spo.x, spo.y, spo.z, __uint_as_float(e));
+    *rb = make_float4(L.x, L.y, L.z, __uint_as_float(li));
+    return true;
+}
+__device__ __forceinline__ void append_ray(const BatchDev& bd, int counter, bool want, float4 ra, float4 rb) {
+    const uint32_t slot = block_append(bd.counters + counter, want);
+    if (want) {
+        bd.qA[slot] = ra;
+        bd.qB[slot] = rb;
+    }
+}
+
 // ---- stage 3: spatial reuse (perPixelSpatialResampling, ris.cl:126-151,
 //      spatialSampling.cl:2-66) -------------------------------------------------------
+// Returns the pixel's reservoir and G-buffer word.
 template <bool POINT>
-__device__ __forceinline__ void spatial_px(const ViewDev* V, int x, int y) {
+__device__ __forceinline__ Res spatial_px(const ViewDev* V, int x, int y, uint2* gout) {
     const Frame& k = V->k;
     const size_t i = (size_t)y * k.W + x;
     const uint4* cA = V->b.cA;
@@ -915,6 +953,7 @@ __device__ __forceinline__ void spatial_px(const ViewDev* V, int x, int y) {
     const uint2* vd = V->b.vd[V->cur];
     Res res = res_load(cA, cB, i);
     const uint2 g = vd[i];
+    *gout = g;
     const uint32_t voxel = g.x & 0x00FFFFFFu;
     if (voxel != 0u && k.spatial) {
         const uint32_t side = g.x >> 24;
@@ -954,27 +993,37 @@ __device__ __forceinline__ void spatial_px(const ViewDev* V, int x, int y) {
         V->b.seed[i] = seed;
     }
     res_store(V->b.hA, V->b.hB, i, res);
+    return res;
 }
 
-template <int VARIANT>
+// LISTS: the pixel's shading request too, from the reservoir at hand (requests_with_spatial).
+template <int VARIANT, bool LISTS>
 __global__ void __launch_bounds__(kMaxTileThreads) spatial_kernel(const __grid_constant__ BatchDev bd) {
     uint32_t tile, round = 0;
     while (next_tile(bd, bd.counters + kCtrSpatial, &tile, round)) {
         int x, y;
         const ViewDev* V = tile_pixel<VARIANT>(bd, tile, &x, &y);
+        bool want = false;
+        float4 ra = make_float4(0.0f, 0.0f, 0.0f, 0.0f), rb = ra;
         if (x < V->k.W && y < V->k.H) {
-            if (point_of<VARIANT>(V)) spatial_px<true>(V, x, y);
-            else spatial_px<false>(V, x, y);
+            uint2 g;
+            const Res r = point_of<VARIANT>(V) ? spatial_px<true>(V, x, y, &g) : spatial_px<false>(V, x, y, &g);
+            if (LISTS && (g.x & 0x00FFFFFFu) != 0u) {
+                const uint32_t v = VARIANT < 2 ? 0u : (uint32_t)(V - bd.views);
+                want = shade_ray(V, (v << 27) | ((uint32_t)y * (uint32_t)V->k.W + (uint32_t)x), x, y, g, r.idx, r.M, r.sumW,
+                                 r.pHat, r.pos, &ra, &rb);
+            }
         }
+        if (LISTS) append_ray(bd, kCtrQ2, want, ra, rb);
     }
 }
 
 // ---- stage 4: shading (renderRIS / render_di_ris, ris.cl:155-293, 391-413) ------------------
-// 4a: a shadow-ray request for every hit pixel whose reservoir has W > 0 and M > 0.
+// (small whole frames append their requests in the spatial pass instead)
 template <int VARIANT>
 __global__ void __launch_bounds__(128) shade_request_kernel(const __grid_constant__ BatchDev bd) {
     const uint32_t nh = bd.counters[kCtrHits];
-    // every thread of a block runs the same iterations (block_append needs all of them)
+    // every thread of a block runs the same iterations (append_ray needs all of them)
     for (uint32_t j0 = blockIdx.x * blockDim.x; j0 < nh; j0 += gridDim.x * blockDim.x) {
         const uint32_t j = j0 + threadIdx.x;
         bool want = false;
@@ -982,35 +1031,12 @@ __global__ void __launch_bounds__(128) shade_request_kernel(const __grid_constan
         if (j < nh) {
             const uint32_t e = bd.hits[j];
             const ViewDev* V = view_of<VARIANT>(bd, e >> 27);
-            const Frame& k = V->k;
             const uint32_t i = pix_of<VARIANT>(e);
-            const uint4 qa = V->b.hA[i];
-            const uint32_t M = qa.y & 0x1FFFFFFFu;
-            const float W = __uint_as_float(qa.z) / fmaxf(1e-5f, __uint_as_float(qa.w) * (float)M);
-            if (W > 0.0f && M > 0u) {
-                const int x = (int)(i % (uint32_t)k.W), y = (int)(i / (uint32_t)k.W);
-                const uint2 g = V->b.vd[V->cur][i];
-                const uint32_t side = g.x >> 24;
-                const float dist = __uint_as_float(g.y);
-                const float3 D = camera_ray(k, x, y);
-                const float nsign = side_sign(side, D);
-                const float3 sp = f3(D.x * dist + k.E.x, D.y * dist + k.E.y, D.z * dist + k.E.z);
-                const float3 spo = f3(sp.x + (side == 0 ? 0.1f * nsign : 0.0f), sp.y + (side == 1 ? 0.1f * nsign : 0.0f),
-                                      sp.z + (side == 2 ? 0.1f * nsign : 0.0f));
-                uint32_t li = qa.x;
-                if (li >= k.nlights) { raise_error(V->b.err, 8u); li = 0; }
-                const float4 qb = __ldg(V->b.hB + i);
-                const float3 L = normalize3(sub(f3(qb.x, qb.y, qb.z), spo));
-                ra = make_float4(spo.x, spo.y, spo.z, __uint_as_float(e));
-                rb = make_float4(L.x, L.y, L.z, __uint_as_float(li));
-                want = true;
-            }
+            const Res r = res_load(V->b.hA, V->b.hB, i);
+            want = shade_ray(V, e, (int)(i % (uint32_t)V->k.W), (int)(i / (uint32_t)V->k.W), V->b.vd[V->cur][i], r.idx, r.M,
+                             r.sumW, r.pHat, r.pos, &ra, &rb);
         }
-        const uint32_t slot = block_append(bd.counters + kCtrQ2, want);
-        if (want) {
-            bd.qA[slot] = ra;
-            bd.qB[slot] = rb;
-        }
+        append_ray(bd, kCtrQ2, want, ra, rb);
     }
 }
 
@@ -1246,7 +1272,7 @@ static void launch_tiles(K kernel, const BatchDev& bd, int ctr, cudaStream_t s, 
     const int threads = bd.tx * bd.ty;
     unsigned nb = std::max(1u, bd.totalTiles);
     if (bd.persistent) {
-        cudaMemsetAsync(bd.counters + ctr, 0, sizeof(uint32_t), s);
+        if (!bd.lists) cudaMemsetAsync(bd.counters + ctr, 0, sizeof(uint32_t), s);
         nb = std::max(1u, std::min(resident_blocks((const void*)kernel, threads), bd.totalTiles));
     }
     Timed tm(bd, id, s);
@@ -1315,8 +1341,15 @@ void launch_path_trace(const BatchDev& bd, cudaStream_t s) {
 }
 
 void launch_batch_albedo(const BatchDev& bd, int variant, cudaStream_t s) {
-    if (variant == 2) launch_tiles(dev::albedo_kernel<2>, bd, kCtrAlbedo, s, K_ALBEDO);
-    else launch_tiles(dev::albedo_kernel<0>, bd, kCtrAlbedo, s, K_ALBEDO);
+    if (bd.lists) {
+        // all of the frame's list lengths and cursors at once
+        cudaMemsetAsync(bd.counters, 0, kCounters * sizeof(uint32_t), s);
+        if (variant == 2) launch_tiles(dev::albedo_kernel<2, true>, bd, kCtrAlbedo, s, K_ALBEDO);
+        else launch_tiles(dev::albedo_kernel<0, true>, bd, kCtrAlbedo, s, K_ALBEDO);
+    } else {
+        if (variant == 2) launch_tiles(dev::albedo_kernel<2, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        else launch_tiles(dev::albedo_kernel<0, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+    }
 }
 
 constexpr int kShadowMinBlocks = 7;   // of shadow_kernel: 728 us against 768 at 6 and 755 at 8 (see there)
@@ -1377,10 +1410,9 @@ template <int VARIANT>
 static void candidates_v(const BatchDev& bd, const LearnedHook* learned, cudaStream_t s, cudaStream_t tail,
                          cudaEvent_t ev) {
     const size_t n = bd.totalPixels;
-    cudaMemsetAsync(bd.counters + kCtrHits, 0, 3 * sizeof(uint32_t), s);   // hits, q1 requests, q1 fetch
-    uint32_t maxPx = VARIANT < 2 ? bd.totalPixels : 0;
-    if (VARIANT == 2) maxPx = (uint32_t)(n / bd.nviews + 1);
-    {
+    if (!bd.lists) {
+        cudaMemsetAsync(bd.counters + kCtrHits, 0, 3 * sizeof(uint32_t), s);   // hits, q1 requests, q1 fetch
+        const uint32_t maxPx = VARIANT < 2 ? bd.totalPixels : (uint32_t)(n / bd.nviews + 1);
         Timed tm(bd, K_COMPACT, s);
         dev::compact_hits_kernel<VARIANT><<<dim3(list_blocks(maxPx, 256, 8), bd.nviews), 256, 0, s>>>(bd);
     }
@@ -1442,16 +1474,29 @@ void launch_batch_candidates(const BatchDev& bd, int variant, const LearnedHook*
     else candidates_v<2>(bd, nullptr, s, tail, ev);
 }
 
+// A whole frame's shading requests come from the spatial pass while the frame is small: that
+// saves a launch and a pass (333 x 187: 265 -> 260 us a frame, 640 x 360: 372 -> 366). From a
+// million pixels on the separate kernel costs less, as it runs beside the next frame's
+// primary rays and the spatial pass keeps its registers (1280 x 720: 15 us a frame less, 1080p
+// 15 us). The line lies between the sizes measured.
+constexpr uint32_t kSpatialRequests = 1u << 19;
+static bool requests_with_spatial(const BatchDev& bd) { return bd.lists && bd.totalPixels <= kSpatialRequests; }
+
+template <bool LISTS>
+static void spatial_v(const BatchDev& bd, int variant, cudaStream_t s) {
+    if (variant == 0) launch_tiles(dev::spatial_kernel<0, LISTS>, bd, kCtrSpatial, s, K_SPATIAL);
+    else if (variant == 1) launch_tiles(dev::spatial_kernel<1, LISTS>, bd, kCtrSpatial, s, K_SPATIAL);
+    else launch_tiles(dev::spatial_kernel<2, LISTS>, bd, kCtrSpatial, s, K_SPATIAL);
+}
 void launch_batch_spatial(const BatchDev& bd, int variant, cudaStream_t s) {
-    if (variant == 0) launch_tiles(dev::spatial_kernel<0>, bd, kCtrSpatial, s, K_SPATIAL);
-    else if (variant == 1) launch_tiles(dev::spatial_kernel<1>, bd, kCtrSpatial, s, K_SPATIAL);
-    else launch_tiles(dev::spatial_kernel<2>, bd, kCtrSpatial, s, K_SPATIAL);
+    if (requests_with_spatial(bd)) spatial_v<true>(bd, variant, s);
+    else spatial_v<false>(bd, variant, s);
 }
 
 template <int VARIANT>
 static void shade_v(const BatchDev& bd, cudaStream_t s) {
-    cudaMemsetAsync(bd.counters + kCtrQ2, 0, 2 * sizeof(uint32_t), s);   // q2 requests, q2 fetch
-    {
+    if (!requests_with_spatial(bd)) {
+        if (!bd.lists) cudaMemsetAsync(bd.counters + kCtrQ2, 0, 2 * sizeof(uint32_t), s);   // q2 requests, q2 fetch
         Timed tm(bd, K_SHADE_REQ, s);
         dev::shade_request_kernel<VARIANT < 2 ? 0 : 2><<<list_blocks(bd.totalPixels, 128, bd.listPerSm), 128, 0, s>>>(bd);
     }

@@ -170,7 +170,8 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     b.counters = (uint32_t*)(s + kOffErr + 64);
     const bool point = light_model == VXR_LIGHTS_POINT;
     const vxr::Tuning sh;
-    const vxr::BatchDev bd = vxr::single_batch(w, f, b, 0, point, sh);
+    vxr::BatchDev bd = vxr::single_batch(w, f, b, 0, point, sh);
+    bd.lists = 1;
     const int variant = point ? 1 : 0;
     vxr::launch_batch_albedo(bd, variant, st);
     vxr::launch_batch_candidates(bd, variant, nullptr, st);

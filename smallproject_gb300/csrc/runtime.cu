@@ -280,15 +280,13 @@ void free_view(vxr_view* v) {
     v->prop = nullptr;
     delete v->ktimer;
     v->ktimer = nullptr;
-    for (int i = 0; i < 6; i++) {
-        if (v->evs[i]) cudaEventDestroy(v->evs[i]);
-        if (v->eve[i]) cudaEventDestroy(v->eve[i]);
-    }
+    if (v->evs) cudaEventDestroy(v->evs);
+    if (v->eve) cudaEventDestroy(v->eve);
     for (cudaEvent_t e : v->ringS) cudaEventDestroy(e);
     for (cudaEvent_t e : v->ringE) cudaEventDestroy(e);
     for (cudaEvent_t e : v->imgEv)
         if (e) cudaEventDestroy(e);
-    for (cudaEvent_t e : {v->evSpatial, v->evFront, v->evNow})
+    for (cudaEvent_t e : {v->evFront, v->evNow})
         if (e) cudaEventDestroy(e);
     if (v->stream2) cudaStreamDestroy(v->stream2);
     if (v->stream) cudaStreamDestroy(v->stream);
@@ -304,7 +302,7 @@ void harvest(vxr_view* v) {
             const int i = slot * 6 + s;
             if (!v->ringUsed[i]) continue;
             float ms = 0.0f;
-            if (cudaEventElapsedTime(&ms, v->ringS[i], v->ringE[i]) == cudaSuccess) {
+            if (cudaEventElapsedTime(&ms, v->ringFrom[i], v->ringE[i]) == cudaSuccess) {
                 v->statSum[s] += ms;
                 v->statCount[s]++;
             }
@@ -545,20 +543,19 @@ int vxr_view_create(vxr_world* w, const vxr_view_desc* d, vxr_view** out) {
     if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&leastPrio, &greatestPrio);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&v->stream, cudaStreamNonBlocking, greatestPrio);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&v->stream2, cudaStreamNonBlocking, greatestPrio);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v->evSpatial, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v->evFront, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v->evNow, cudaEventDisableTiming);
     v->ringS.assign(vxr_view::kRing * 6, nullptr);
     v->ringE.assign(vxr_view::kRing * 6, nullptr);
+    v->ringFrom.assign(vxr_view::kRing * 6, nullptr);
     v->ringUsed.assign(vxr_view::kRing * 6, 0);
+    std::fill(std::begin(v->ran), std::end(v->ran), -1);
     for (int i = 0; i < vxr_view::kRing * 6 && e == cudaSuccess; i++) {
         e = cudaEventCreate(&v->ringS[i]);
         if (e == cudaSuccess) e = cudaEventCreate(&v->ringE[i]);
     }
-    for (int i = 0; i < 6 && e == cudaSuccess; i++) {
-        e = cudaEventCreate(&v->evs[i]);
-        if (e == cudaSuccess) e = cudaEventCreate(&v->eve[i]);
-    }
+    if (e == cudaSuccess) e = cudaEventCreate(&v->evs);
+    if (e == cudaSuccess) e = cudaEventCreate(&v->eve);
     if (e != cudaSuccess) {
         free_view(v);
         delete v;
@@ -684,7 +681,7 @@ int vxr_view_begin_frame(vxr_view* v, vxr_frame_consts* out) {
     std::swap(v->buf.counters, v->buf.countersAlt);
     if (int r = vxr::brick_cache_begin(v)) return r;
     v->frameOpen = true;
-    for (int i = 0; i < 6; i++) v->ran[i] = false;
+    std::fill(std::begin(v->ran), std::end(v->ran), -1);
     if (out) *out = k;
     return VXR_OK;
 }
@@ -700,7 +697,8 @@ int vxr_view_set_frame_consts(vxr_view* v, const vxr_frame_consts* k) {
     return VXR_OK;
 }
 
-// s: the stream of the stage's launches; tail (candidate stage): the stream of its
+// fuse: a whole frame's stage (shading accumulates; lists filled by the kernels before them,
+// unless kernels are timed one by one). s: the stream of the stage's launches; tail (candidate stage): the stream of its
 // temporal pass, handed on by an event (null: s)
 static int run_stage(vxr_view* v, int stage, bool fuse, cudaStream_t s, cudaStream_t tail = nullptr) {
     if (!tail) tail = s;
@@ -718,11 +716,17 @@ static int run_stage(vxr_view* v, int stage, bool fuse, cudaStream_t s, cudaStre
         return VXR_OK;
     }
     const int ri = (int)(v->frameSerial % vxr_view::kRing) * 6 + stage;
-    CUV(cudaEventRecord(v->evs[stage], s), "cudaEventRecord");
-    CUV(cudaEventRecord(v->ringS[ri], s), "cudaEventRecord");
+    // in a whole frame the stage before ended on this stream just now
+    if (fuse && stage > VXR_STAGE_ALBEDO) {
+        v->ringFrom[ri] = v->ringE[ri - 1];
+    } else {
+        CUV(cudaEventRecord(v->ringS[ri], s), "cudaEventRecord");
+        v->ringFrom[ri] = v->ringS[ri];
+    }
     vxr::BatchDev bd = vxr::single_batch(w, k, v->buf, v->cur, point, sh);
     bd.fuse = fuse ? 1 : 0;
     bd.timer = v->ktimerOn ? v->ktimer : nullptr;
+    bd.lists = fuse && !bd.timer ? 1 : 0;
     if (sh.brickCache > 0) {
         if (v->bc.calibrating) {
             bd.bcCount = v->bc.count;
@@ -747,10 +751,9 @@ static int run_stage(vxr_view* v, int stage, bool fuse, cudaStream_t s, cudaStre
     default: return set_error(VXR_E_INVALID, "vxr_view_stage: unknown stage");
     }
     CUV(cudaGetLastError(), "kernel launch");
-    CUV(cudaEventRecord(v->eve[stage], tail), "cudaEventRecord");
     CUV(cudaEventRecord(v->ringE[ri], tail), "cudaEventRecord");
     v->ringUsed[ri] = 1;
-    v->ran[stage] = true;
+    v->ran[stage] = ri;
     return VXR_OK;
 }
 
@@ -782,10 +785,10 @@ int vxr_view_render(vxr_view* v) {
     if (int r = vxr_view_begin_frame(v, nullptr)) return r;
     if (!overlap) CUV(cudaEventRecord(v->evNow, v->stream), "cudaEventRecord");
     CUV(cudaStreamWaitEvent(v->stream2, overlap ? v->evSpatial : v->evNow, 0), "cudaStreamWaitEvent");
-    if (int r = run_stage(v, VXR_STAGE_ALBEDO, false, v->stream2)) return r;
-    if (int r = run_stage(v, VXR_STAGE_CANDIDATES, false, v->stream2, v->stream)) return r;
-    if (int r = run_stage(v, VXR_STAGE_SPATIAL, false, v->stream)) return r;
-    CUV(cudaEventRecord(v->evSpatial, v->stream), "cudaEventRecord");
+    if (int r = run_stage(v, VXR_STAGE_ALBEDO, true, v->stream2)) return r;
+    if (int r = run_stage(v, VXR_STAGE_CANDIDATES, true, v->stream2, v->stream)) return r;
+    if (int r = run_stage(v, VXR_STAGE_SPATIAL, true, v->stream)) return r;
+    v->evSpatial = v->ringE[v->ran[VXR_STAGE_SPATIAL]];
     if (int r = run_stage(v, VXR_STAGE_SHADE, true, v->stream)) return r;
     if (int r = vxr::proposal_frame_train(v)) return r;
     if (int r = vxr_view_end_frame(v)) return r;
@@ -801,7 +804,7 @@ static int view_wait(vxr_view* v, bool join) {
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_wait");
     for (int s = 1; s <= 5; s++) {
         float ms = 0.0f;
-        if (v->ran[s]) cudaEventElapsedTime(&ms, v->evs[s], v->eve[s]);
+        if (v->ran[s] >= 0) cudaEventElapsedTime(&ms, v->ringFrom[v->ran[s]], v->ringE[v->ran[s]]);
         v->times[s - 1] = ms;
     }
     harvest(v);
@@ -1039,7 +1042,7 @@ int vxr_host_free(void* p) {
 int vxr_view_timer_begin(vxr_view* v) {
     if (int r = check_view(v, "vxr_view_timer_begin")) return r;
     v->spatialEvOk = false;   // the next frame's primary rays start after this mark
-    CUV(cudaEventRecord(v->evs[0], v->stream), "cudaEventRecord");
+    CUV(cudaEventRecord(v->evs, v->stream), "cudaEventRecord");
     return VXR_OK;
 }
 
@@ -1047,9 +1050,9 @@ int vxr_view_timer_end(vxr_view* v, float* ms) {
     if (int r = check_view(v, "vxr_view_timer_end")) return r;
     VXR_CHECK_ARG(ms, "vxr_view_timer_end: null output");
     vxr::proposal_join(v);   // the timed region ends after the last frame's training step
-    CUV(cudaEventRecord(v->eve[0], v->stream), "cudaEventRecord");
-    CUV(cudaEventSynchronize(v->eve[0]), "cudaEventSynchronize");
-    CUV(cudaEventElapsedTime(ms, v->evs[0], v->eve[0]), "cudaEventElapsedTime");
+    CUV(cudaEventRecord(v->eve, v->stream), "cudaEventRecord");
+    CUV(cudaEventSynchronize(v->eve), "cudaEventSynchronize");
+    CUV(cudaEventElapsedTime(ms, v->evs, v->eve), "cudaEventElapsedTime");
     return VXR_OK;
 }
 

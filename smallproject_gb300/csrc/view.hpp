@@ -85,13 +85,15 @@ struct vxr_view {
     // (evFront). spatialEvOk: evSpatial marks the last frame's spatial pass and nothing
     // has touched the buffers since.
     cudaStream_t stream2 = nullptr;
-    cudaEvent_t evSpatial = nullptr, evFront = nullptr, evNow = nullptr;
+    cudaEvent_t evSpatial = nullptr, evFront = nullptr, evNow = nullptr;   // (evSpatial: one of ringE)
     bool spatialEvOk = false;
-    cudaEvent_t evs[6] = {}, eve[6] = {};            // [0]: vxr_view_timer_*, [1..5]: last frame's stages
-    bool ran[6] = {};
-    // per-stage event ring over the last kRing frames, harvested by vxr_view_wait
+    cudaEvent_t evs = nullptr, eve = nullptr;         // vxr_view_timer_*
+    int ran[6] = {};                                  // per stage: its ring entry in the last frame that ran it, -1 none
+    // per-stage event ring over the last kRing frames, harvested by vxr_view_wait; a stage of
+    // a whole frame starts where the one before it ends, with that one's end event
     static constexpr int kRing = 256;
     std::vector<cudaEvent_t> ringS, ringE;             // kRing * 6
+    std::vector<cudaEvent_t> ringFrom;                 // kRing * 6: the event a stage's time starts at
     std::vector<uint8_t> ringUsed;                     // kRing * 6
     uint64_t frameSerial = 0, harvested = 0;
     double statSum[6] = {};
