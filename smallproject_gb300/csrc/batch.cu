@@ -351,13 +351,8 @@ int vxr_batch_wait(vxr_batch* b, float* ms) {
     }
     uint32_t any = 0;
     for (vxr_view* v : b->views) {
-        uint32_t err = 0;
-        e = cudaMemcpy(&err, v->buf.err, sizeof(err), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return cuda_error(e, "vxr_batch_wait: read device error flags");
-        if (err) {
-            cudaMemset(v->buf.err, 0, sizeof(uint32_t));
-            any |= err;
-        }
+        any |= *v->errHost;
+        *v->errHost = 0u;
     }
     if (any)
         return vxr::set_error(VXR_E_DEVICE, vxr::device_flags_message(any));

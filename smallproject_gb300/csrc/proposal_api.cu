@@ -737,10 +737,8 @@ int vxr_view_proposal_probs(vxr_view* v, uint32_t n, const float* samples, float
     a.err = v->buf.err;
     cudaError_t e = vxr::prop::launch_infer(a, n, v->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(v->stream);
-    uint32_t flags = 0;
-    if (e == cudaSuccess) e = cudaMemcpy(&flags, v->buf.err, sizeof(flags), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && (flags & 16u)) {
-        cudaMemset(v->buf.err, 0, sizeof(uint32_t));
+    if (e == cudaSuccess && (*v->errHost & 16u)) {
+        *v->errHost = 0u;
         cudaFree(ds);
         cudaFree(dp);
         return set_error(VXR_E_DEVICE, "vxr_view_proposal_probs: a tensor-core wait gave up");

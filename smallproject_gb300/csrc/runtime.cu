@@ -270,7 +270,7 @@ void free_view(vxr_view* v) {
     vxr::ViewBuffers& b = v->buf;
     cudaFree(b.vd[0]); cudaFree(b.vd[1]); cudaFree(b.seed);
     cudaFree(b.cA); cudaFree(b.cB); cudaFree(b.hA); cudaFree(b.hB);
-    cudaFree(b.frame); cudaFree(b.accum); cudaFree(b.err);
+    cudaFree(b.frame); cudaFree(b.accum); cudaFreeHost((void*)v->errHost);
     cudaFree(b.hits); cudaFree(b.qA); cudaFree(b.qB); cudaFree(b.counters);
     cudaFree(b.hitsAlt); cudaFree(b.qAAlt); cudaFree(b.qBAlt); cudaFree(b.countersAlt);
     cudaFree(v->sum64); cudaFree(v->errOut);
@@ -292,11 +292,11 @@ void free_view(vxr_view* v) {
     if (v->stream) cudaStreamDestroy(v->stream);
 }
 
-// Accumulate the stage durations of every finished frame still in the ring.
-void harvest(vxr_view* v) {
+// Accumulate the stage durations of the frames before `upto` (finished ones) still in the ring.
+void harvest(vxr_view* v, uint64_t upto) {
     const uint64_t from = v->frameSerial > (uint64_t)vxr_view::kRing ? std::max(v->harvested, v->frameSerial - vxr_view::kRing)
                                                                        : v->harvested;
-    for (uint64_t f = from; f < v->frameSerial; f++) {
+    for (uint64_t f = from; f < upto; f++) {
         const int slot = (int)(f % vxr_view::kRing);
         for (int s = 1; s <= 5; s++) {
             const int i = slot * 6 + s;
@@ -309,7 +309,26 @@ void harvest(vxr_view* v) {
             v->ringUsed[i] = 0;
         }
     }
-    v->harvested = v->frameSerial;
+    v->harvested = std::max(v->harvested, upto);
+}
+
+// the stage times of the last waited frame, from its ring entries
+void settle_times(vxr_view* v) {
+    if (!v->timesDue) return;
+    v->timesDue = false;
+    for (int s = 1; s <= 5; s++) {
+        const int ri = v->waitedRan[s];
+        v->times[s - 1] = 0.0f;
+        if (ri >= 0) cudaEventElapsedTime(&v->times[s - 1], v->ringFrom[ri], v->ringE[ri]);
+    }
+}
+
+// the view's device error flags, reported once
+int report_flags(vxr_view* v) {
+    const uint32_t err = *v->errHost;
+    if (!err) return VXR_OK;
+    *v->errHost = 0u;
+    return set_error(VXR_E_DEVICE, device_flags_message(err));
 }
 
 void ViewKernelTimer::mark(int k, bool end, cudaStream_t s) {
@@ -528,7 +547,9 @@ int vxr_view_create(vxr_world* w, const vxr_view_desc* d, vxr_view** out) {
     alloc((void**)&b.hB, n * sizeof(float4));
     alloc((void**)&b.frame, n * sizeof(float4));
     alloc((void**)&b.accum, n * sizeof(float4));
-    alloc((void**)&b.err, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&v->errHost, sizeof(uint32_t), cudaHostAllocMapped);
+    if (e == cudaSuccess) *v->errHost = 0u;
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&b.err, (void*)v->errHost, 0);
     alloc((void**)&b.hits, n * sizeof(uint32_t));
     alloc((void**)&b.qA, n * sizeof(float4));
     alloc((void**)&b.qB, n * sizeof(float4));
@@ -550,6 +571,7 @@ int vxr_view_create(vxr_world* w, const vxr_view_desc* d, vxr_view** out) {
     v->ringFrom.assign(vxr_view::kRing * 6, nullptr);
     v->ringUsed.assign(vxr_view::kRing * 6, 0);
     std::fill(std::begin(v->ran), std::end(v->ran), -1);
+    std::fill(std::begin(v->waitedRan), std::end(v->waitedRan), -1);
     for (int i = 0; i < vxr_view::kRing * 6 && e == cudaSuccess; i++) {
         e = cudaEventCreate(&v->ringS[i]);
         if (e == cudaSuccess) e = cudaEventCreate(&v->ringE[i]);
@@ -680,6 +702,9 @@ int vxr_view_begin_frame(vxr_view* v, vxr_frame_consts* out) {
     std::swap(v->buf.qB, v->buf.qBAlt);
     std::swap(v->buf.counters, v->buf.countersAlt);
     if (int r = vxr::brick_cache_begin(v)) return r;
+    // the ring slot this frame takes may hold a waited frame whose times are not worked out yet
+    if (v->frameSerial + 1 - v->waitedSerial >= (uint64_t)vxr_view::kRing) vxr::settle_times(v);
+    if (v->frameSerial - v->harvested >= (uint64_t)vxr_view::kRing && v->harvested < v->waitedSerial) harvest(v, v->waitedSerial);
     v->frameOpen = true;
     std::fill(std::begin(v->ran), std::end(v->ran), -1);
     if (out) *out = k;
@@ -802,22 +827,14 @@ int vxr_view_render(vxr_view* v) {
 static int view_wait(vxr_view* v, bool join) {
     if (join) vxr::proposal_join(v);
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_wait");
-    for (int s = 1; s <= 5; s++) {
-        float ms = 0.0f;
-        if (v->ran[s] >= 0) cudaEventElapsedTime(&ms, v->ringFrom[v->ran[s]], v->ringE[v->ran[s]]);
-        v->times[s - 1] = ms;
-    }
-    harvest(v);
+    // (stage times are worked out when they are asked for, or when the ring comes round)
+    std::copy(std::begin(v->ran), std::end(v->ran), v->waitedRan);
+    v->timesDue = true;
+    v->waitedSerial = v->frameSerial;
     // kernel times once every marked kernel has run (the training step's marks are on its
     // side stream)
     if (v->ktimer && join) v->ktimer->harvest();
-    uint32_t err = 0;
-    CUV(cudaMemcpy(&err, v->buf.err, sizeof(err), cudaMemcpyDeviceToHost), "read device error flags");
-    if (err) {
-        cudaMemset(v->buf.err, 0, sizeof(uint32_t));
-        return set_error(VXR_E_DEVICE, vxr::device_flags_message(err));
-    }
-    return VXR_OK;
+    return vxr::report_flags(v);
 }
 
 int vxr_view_wait(vxr_view* v) {
@@ -828,6 +845,7 @@ int vxr_view_wait(vxr_view* v) {
 int vxr_view_stage_times(vxr_view* v, float ms[5]) {
     if (int r = check_view(v, "vxr_view_stage_times")) return r;
     VXR_CHECK_ARG(ms, "vxr_view_stage_times: null output");
+    vxr::settle_times(v);
     for (int i = 0; i < 5; i++) ms[i] = v->times[i];
     return VXR_OK;
 }
@@ -972,13 +990,7 @@ int vxr_view_image_wait(vxr_view* v, uint64_t ticket) {
     VXR_CHECK_ARG(ticket < v->imgSerial && v->imgSerial - ticket <= (uint64_t)vxr_view::kImages,
                   "vxr_view_image_wait: unknown or expired ticket");
     CUV(cudaEventSynchronize(v->imgEv[ticket % vxr_view::kImages]), "vxr_view_image_wait");
-    uint32_t err = 0;
-    CUV(cudaMemcpy(&err, v->buf.err, sizeof(err), cudaMemcpyDeviceToHost), "read device error flags");
-    if (err) {
-        cudaMemset(v->buf.err, 0, sizeof(uint32_t));
-        return set_error(VXR_E_DEVICE, vxr::device_flags_message(err));
-    }
-    return VXR_OK;
+    return vxr::report_flags(v);
 }
 
 }  // extern "C"
@@ -1215,7 +1227,8 @@ extern "C" int vxr_view_stage_stats(vxr_view* v, double sum_ms[5], uint32_t coun
     if (int r = check_view(v, "vxr_view_stage_stats")) return r;
     VXR_CHECK_ARG(sum_ms && count, "vxr_view_stage_stats: null output");
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_stage_stats");
-    harvest(v);
+    v->waitedSerial = v->frameSerial;
+    harvest(v, v->frameSerial);
     for (int s = 1; s <= 5; s++) {
         sum_ms[s - 1] = v->statSum[s];
         count[s - 1] = v->statCount[s];

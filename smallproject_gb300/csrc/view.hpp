@@ -116,7 +116,13 @@ struct vxr_view {
     bool frameOpen = false;
     vxr_frame_consts k{};
     uint64_t seenLightVersion = 0, seenLightMoveVersion = 0;
-    float times[5] = {};
+    int waitedRan[6] = {};                            // `ran` of the last waited frame,
+    float times[5] = {};                              // its stage times,
+    bool timesDue = false;                            // still to be worked out
+    uint64_t waitedSerial = 0;                        // frames before it have been waited for
+    // device error flags, in page-locked memory the kernels write through buf.err: reading them
+    // after a wait is a load
+    volatile uint32_t* errHost = nullptr;
     size_t npx = 0;
 };
 
@@ -127,7 +133,8 @@ dev::World dev_world(vxr_view* v);
 dev::Frame dev_frame(const vxr_frame_consts& c);
 int ensure_world(vxr_view* v);
 void free_view(vxr_view* v);
-void harvest(vxr_view* v);
+void harvest(vxr_view* v, uint64_t upto);
+int report_flags(vxr_view* v);
 Tuning shape(const vxr_view* v);
 int check_tuning(const vxr_tuning* t, const char* fn);
 Tuning to_tuning(const vxr_tuning& t);
