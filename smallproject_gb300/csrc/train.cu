@@ -39,7 +39,8 @@ namespace prop {
 
 namespace {
 
-constexpr int kTW = 8;          // warps per CTA
+constexpr int kTW = 8;          // warps per CTA of wgrad_kernel
+constexpr int kTrainWarps = 8;  // and of train_kernel (9 to 16 at fewer registers: 64 to 71 us a batch of 65,536 against 63)
 constexpr int kTrainCtasPerSm = 1;   // train_kernel: one CTA per SM (two, capped at 128 registers, spill and run slower)
 constexpr int kTH = 64;         // hidden width handled by the fused step
 constexpr int kLd1 = kIn + 8;   // padded row of W1 and X in shared memory (BF16 elements)
@@ -155,6 +156,24 @@ __device__ __forceinline__ void logits_tile(float (&c)[4], const uint32_t (&h3)[
     }
 }
 
+// Table entries and trilinear weights of the 8 corners of point p on level l, as
+// level_features takes them.
+__device__ __forceinline__ void level_corners(const Dims& d, float4 p, int l, uint32_t (&idx)[8], float (&w)[8]) {
+    const uint32_t mask = (1u << d.tableLog2) - 1u;
+    const int R = l == 0 ? d.res0 : d.res1;
+    const float s = (float)R * (1.0f / 1024.0f);
+    const float ux = fminf(fmaxf(p.x * s, 0.0f), (float)R), uy = fminf(fmaxf(p.y * s, 0.0f), (float)R),
+                uz = fminf(fmaxf(p.z * s, 0.0f), (float)R);
+    const int ix = min((int)ux, R - 1), iy = min((int)uy, R - 1), iz = min((int)uz, R - 1);
+    const float fx = ux - (float)ix, fy = uy - (float)iy, fz = uz - (float)iz;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int ox = q & 1, oy = (q >> 1) & 1, oz = q >> 2;
+        idx[q] = (uint32_t)l * (mask + 1u) + grid_hash((uint32_t)(ix + ox), (uint32_t)(iy + oy), (uint32_t)(iz + oz), mask);
+        w[q] = (ox ? fx : 1.0f - fx) * (oy ? fy : 1.0f - fy) * (oz ? fz : 1.0f - fz);
+    }
+}
+
 __global__ void wsum_kernel(const float* __restrict__ w, uint32_t B, float* __restrict__ part) {
     __shared__ float ws[8];
     float s = 0.0f;
@@ -170,10 +189,13 @@ __global__ void wsum_kernel(const float* __restrict__ w, uint32_t B, float* __re
     }
 }
 
-__global__ void __launch_bounds__(kTW * 32, kTrainCtasPerSm) train_kernel(TrainArgs a) {
+// 65,536 samples, 256 clusters: 63 us, 94 with the weights staged 2 bytes a copy (27 us of them)
+// and a lane per table entry (4 us). The load and store pipe is the busiest (59 % of its
+// wavefronts while active: the mma operands from shared memory), more warps do not help.
+__global__ void __launch_bounds__(kTrainWarps * 32, kTrainCtasPerSm) train_kernel(TrainArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float s_inv;
-    __shared__ float s_loss[kTW];
+    __shared__ float s_loss[kTrainWarps];
     const Dims d = a.dims;
     const int K = d.K, kt4 = K / 16;
     __nv_bfloat16* W1s = reinterpret_cast<__nv_bfloat16*>(smem);   // [64][40]
@@ -183,19 +205,19 @@ __global__ void __launch_bounds__(kTW * 32, kTrainCtasPerSm) train_kernel(TrainA
     float* bs = reinterpret_cast<float*>(W4s + K * kLdh);            // b1 | b2 | b3 | b4
     unsigned char* wbase = reinterpret_cast<unsigned char*>(bs + 3 * kTH + K);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int r = lane & 15, half = lane >> 4;
+    const int r = lane >> 1, half = lane & 1;
     __nv_bfloat16* Xs = reinterpret_cast<__nv_bfloat16*>(wbase + warp * kTrainWarpBytes);   // [16][40]
     __nv_bfloat16* H1s = Xs + 16 * kLd1;                                                   // [16][72]
     float* dxs = reinterpret_cast<float*>(H1s + 16 * kLdh);                                // [16][16]
     {
-        const __nv_bfloat16* wg = a.wbf;   // W1 [64][32] | W2 [64][64] | W3 [64][64] | W4 [K][64]
-        for (int e = threadIdx.x; e < kTH * kIn; e += blockDim.x) W1s[(e / kIn) * kLd1 + e % kIn] = wg[e];
-        wg += kTH * kIn;
-        for (int e = threadIdx.x; e < kTH * kTH; e += blockDim.x) W2s[(e / kTH) * kLdh + e % kTH] = wg[e];
-        wg += kTH * kTH;
-        for (int e = threadIdx.x; e < kTH * kTH; e += blockDim.x) W3s[(e / kTH) * kLdh + e % kTH] = wg[e];
-        wg += kTH * kTH;
-        for (int e = threadIdx.x; e < K * kTH; e += blockDim.x) W4s[(e / kTH) * kLdh + e % kTH] = wg[e];
+        // W1 [64][32] | W2 [64][64] | W3 [64][64] | W4 [K][64], 8 elements (16 bytes) a copy
+        const uint4* wg = reinterpret_cast<const uint4*>(a.wbf);
+        for (int e = threadIdx.x; e < kTH * kIn / 8; e += blockDim.x)
+            *reinterpret_cast<uint4*>(W1s + (e / (kIn / 8)) * kLd1 + e % (kIn / 8) * 8) = wg[e];
+        wg += kTH * kIn / 8;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < (2 * kTH + K) * kTH / 8; e += blockDim.x)
+            *reinterpret_cast<uint4*>(W2s + (e / (kTH / 8)) * kLdh + e % (kTH / 8) * 8) = wg[e];
         const float* p = a.params;
         for (int e = threadIdx.x; e < kTH; e += blockDim.x) {
             bs[e] = p[a.L.b1 + e];
@@ -216,30 +238,38 @@ __global__ void __launch_bounds__(kTW * 32, kTrainCtasPerSm) train_kernel(TrainA
     const float inv = s_inv;
     const float* enc = a.params + a.L.enc;
     float* encGrad = a.grads + a.L.enc;
-    const uint32_t mask = (1u << d.tableLog2) - 1u;
     const uint32_t ntiles = (a.B + 15u) / 16u;
     uint4* frag = a.frag;
     float lossAcc = 0.0f;
-    for (uint32_t tile = blockIdx.x * kTW + warp; tile < ntiles; tile += gridDim.x * kTW) {
+    for (uint32_t tile = blockIdx.x * kTrainWarps + warp; tile < ntiles; tile += gridDim.x * kTrainWarps) {
         const uint32_t base = tile * 16u;
-        // ---- input rows: lane (r, half) encodes level `half` of sample r
+        // ---- input rows: lanes 2r and 2r + 1 encode sample r, four of the eight features of
+        // both levels each, so that the two read a table entry's 32-byte sector together (the
+        // load and store pipe bounds this kernel; a lane per entry asks for every sector twice)
         const uint32_t j = base + (uint32_t)r;
         const bool valid = j < a.B;
         const float4 pin = valid ? a.samples[j] : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(6u));
         {
-            float f[8];
-            level_features(enc, d, pin.x, pin.y, pin.z, half, f);
             __nv_bfloat16* xr = Xs + r * kLd1;
 #pragma unroll
-            for (int q = 0; q < 8; q += 2)
-                *reinterpret_cast<uint32_t*>(xr + half * 8 + q) = valid ? pack_bf16(f[q], f[q + 1]) : 0u;
-            if (half == 0) {
-                const uint32_t code = __float_as_uint(pin.w);
+            for (int l = 0; l < kLevels; l++) {
+                uint32_t idx[8];
+                float w[8], f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                level_corners(d, pin, l, idx, w);
 #pragma unroll
-                for (int q = 16; q < kIn; q += 2)
-                    *reinterpret_cast<uint32_t*>(xr + q) =
-                        valid ? pack_bf16(code == (uint32_t)(q - 16) ? 1.f : 0.f, code == (uint32_t)(q - 15) ? 1.f : 0.f)
-                              : 0u;
+                for (int q = 0; q < 8; q++) {
+                    const float4 e = __ldg(reinterpret_cast<const float4*>(enc + (size_t)idx[q] * kFeat) + half);
+                    f[0] += w[q] * e.x; f[1] += w[q] * e.y; f[2] += w[q] * e.z; f[3] += w[q] * e.w;
+                }
+                *reinterpret_cast<uint2*>(xr + l * 8 + half * 4) =
+                    valid ? make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3])) : make_uint2(0u, 0u);
+            }
+            const uint32_t code = __float_as_uint(pin.w);
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) {
+                const uint32_t c0 = (uint32_t)(half * 8 + q);
+                *reinterpret_cast<uint32_t*>(xr + 16 + c0) =
+                    valid ? pack_bf16(code == c0 ? 1.f : 0.f, code == c0 + 1u ? 1.f : 0.f) : 0u;
             }
         }
         const uint32_t j0 = base + (uint32_t)g, j1 = j0 + 8u;
@@ -383,23 +413,16 @@ __global__ void __launch_bounds__(kTW * 32, kTrainCtasPerSm) train_kernel(TrainA
         }
         __syncwarp();
         if (valid) {
-            const float4 ga = *reinterpret_cast<const float4*>(dxs + r * 16 + half * 8);
-            const float4 gbv = *reinterpret_cast<const float4*>(dxs + r * 16 + half * 8 + 4);
-            const int R = half == 0 ? d.res0 : d.res1;
-            const float sc = (float)R * (1.0f / 1024.0f);
-            const float ux = fminf(fmaxf(pin.x * sc, 0.0f), (float)R), uy = fminf(fmaxf(pin.y * sc, 0.0f), (float)R),
-                        uz = fminf(fmaxf(pin.z * sc, 0.0f), (float)R);
-            const int ix = min((int)ux, R - 1), iy = min((int)uy, R - 1), iz = min((int)uz, R - 1);
-            const float fx = ux - (float)ix, fy = uy - (float)iy, fz = uz - (float)iz;
 #pragma unroll
-            for (int qc = 0; qc < 8; qc++) {
-                const int ox = qc & 1, oy = (qc >> 1) & 1, oz = qc >> 2;
-                const uint32_t idx = (uint32_t)half * (mask + 1u) +
-                                     grid_hash((uint32_t)(ix + ox), (uint32_t)(iy + oy), (uint32_t)(iz + oz), mask);
-                const float w = (ox ? fx : 1.0f - fx) * (oy ? fy : 1.0f - fy) * (oz ? fz : 1.0f - fz);
-                float4* dst = reinterpret_cast<float4*>(encGrad + (size_t)idx * kFeat);
-                atomicAdd(dst, make_float4(w * ga.x, w * ga.y, w * ga.z, w * ga.w));
-                atomicAdd(dst + 1, make_float4(w * gbv.x, w * gbv.y, w * gbv.z, w * gbv.w));
+            for (int l = 0; l < kLevels; l++) {
+                const float4 gv = *reinterpret_cast<const float4*>(dxs + r * 16 + l * 8 + half * 4);
+                uint32_t idx[8];
+                float w[8];
+                level_corners(d, pin, l, idx, w);
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    atomicAdd(reinterpret_cast<float4*>(encGrad + (size_t)idx[q] * kFeat) + half,
+                              make_float4(w[q] * gv.x, w[q] * gv.y, w[q] * gv.z, w[q] * gv.w));
             }
         }
         __syncwarp();
@@ -411,7 +434,7 @@ __global__ void __launch_bounds__(kTW * 32, kTrainCtasPerSm) train_kernel(TrainA
     __syncthreads();
     if (threadIdx.x == 0) {
         float s = 0.0f;
-        for (int w = 0; w < kTW; w++) s += s_loss[w];
+        for (int w = 0; w < kTrainWarps; w++) s += s_loss[w];
         a.lossPart[blockIdx.x] = s;
     }
 }
@@ -529,12 +552,21 @@ __global__ void __launch_bounds__(256) train_reduce_kernel(ReduceArgs r) {
         else if (i >= sW4 && i < sb4) o = H * kIn + 2 * H * H + (i - sW4);
         if (o >= 0) r.wbf[o] = __float2bfloat16_rn(p);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    // the loss and the weight sum, by the first warp (one thread adding 400 numbers in turn took
+    // longer than the rest of the kernel)
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
         float l = 0.0f, w = 0.0f;
-        for (int c = 0; c < r.nloss; c++) l += r.lossPart[c];
-        for (uint32_t c = 0; c < r.nwpart; c++) w += r.wpart[c];
-        r.scal[0] = l;
-        r.scal[1] = w;
+        for (int c = threadIdx.x; c < r.nloss; c += 32) l += r.lossPart[c];
+        for (uint32_t c = threadIdx.x; c < r.nwpart; c += 32) w += r.wpart[c];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            l += __shfl_xor_sync(0xffffffffu, l, o);
+            w += __shfl_xor_sync(0xffffffffu, w, o);
+        }
+        if (threadIdx.x == 0) {
+            r.scal[0] = l;
+            r.scal[1] = w;
+        }
     }
 }
 
@@ -576,7 +608,7 @@ int train_mlp_count(const Dims& d) { return (int)(layout(d).total - layout(d).W1
 
 size_t train_smem_bytes(const Dims& d) {
     return (size_t)(kTH * kLd1 + 2 * kTH * kLdh + d.K * kLdh) * 2 + (size_t)(3 * kTH + d.K) * 4 +
-           (size_t)kTW * kTrainWarpBytes;
+           (size_t)kTrainWarps * kTrainWarpBytes;
 }
 
 size_t train_frag_bytes(const Dims& d, uint32_t B) {
@@ -597,8 +629,8 @@ cudaError_t launch_train(const TrainArgs& a, cudaStream_t s, int* nparts, int* n
     cudaError_t e = cudaFuncSetAttribute(train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     const uint32_t tiles = (a.B + 15) / 16;
-    const int ctas = (int)std::max<uint32_t>(1, std::min<uint32_t>((tiles + kTW - 1) / kTW, (uint32_t)train_max_ctas()));
-    train_kernel<<<ctas, kTW * 32, sm, s>>>(a);
+    const int ctas = (int)std::max<uint32_t>(1, std::min<uint32_t>((tiles + kTrainWarps - 1) / kTrainWarps, (uint32_t)train_max_ctas()));
+    train_kernel<<<ctas, kTrainWarps * 32, sm, s>>>(a);
     *nloss = ctas;
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
