@@ -36,11 +36,12 @@ struct ViewBuffers {
 enum : int {
     kCtrHits = 0,       // hit-list length
     kCtrQ1 = 1,         // candidate shadow queue: [1] requests, [2] fetch cursor
-    kCtrQ2 = 3,         // shading shadow queue:   [3] requests, [4] fetch cursor
-    kCtrFinish = 5,     // tile cursors of the persistent pixel stages
-    kCtrAlbedo = 6,
-    kCtrSpatial = 7,
-    kCtrAccum = 8,
+    kCtrOut1 = 3,       // candidate shadow rays decided without tracing (shadow_can_reach)
+    kCtrQ2 = 4,         // shading shadow queue:   [4] requests, [5] fetch cursor
+    kCtrFinish = 6,     // tile cursors of the persistent pixel stages
+    kCtrAlbedo = 7,
+    kCtrSpatial = 8,
+    kCtrAccum = 9,
     kCounters = 16
 };
 

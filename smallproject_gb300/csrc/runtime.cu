@@ -1211,7 +1211,7 @@ extern "C" int vxr_view_work_counts(vxr_view* v, uint32_t counts[3]) {
     CUV(cudaMemcpyAsync(c, v->buf.counters, sizeof(c), cudaMemcpyDeviceToHost, v->stream), "read counters");
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_work_counts");
     counts[0] = c[vxr::kCtrHits];
-    counts[1] = c[vxr::kCtrQ1];
+    counts[1] = c[vxr::kCtrQ1] + c[vxr::kCtrOut1];   // traced, or decided before the tracer
     counts[2] = c[vxr::kCtrQ2];
     return VXR_OK;
 }

@@ -70,6 +70,11 @@ int dh_shadow_split(const uint32_t* grid, const uint32_t* bricks, const uint32_t
     return ex <= vx && ex + size > vx && ey <= vy && ey + size > vy && ez <= vz && ez + size > vz;
 }
 
+int dh_can_reach(const uint8_t* uber, const float* O, const float* D, uint32_t pos, uint32_t size, int steps) {
+    return shadow_can_reach(uber, f3(O[0], O[1], O[2]), f3(D[0], D[1], D[2]), pos,
+                            size, steps);
+}
+
 // trace_first with a budget, or a primary ray (boxes: gbox0 given)
 uint32_t dh_trace_first(const uint32_t* grid, const uint8_t* uber, const uint32_t* bricks, const uint32_t* ucell0, const uint32_t* gbox0,
                         const float* O, const float* D, int budget, int steps, float* dist, uint32_t* side) {

@@ -145,6 +145,48 @@ def test_split_walk_finds_solid_cells(dh, split):  # noqa: F811
     assert hits > 300
 
 
+def _compare_reach(dh, split, wa, O, D, pos, size):  # noqa: F811
+    """Rays shadow_can_reach rules out are occluded for the walker; returns (rays, ruled out,
+    visible)."""
+    boxes = brick_boxes(wa.bricks)
+    P = lambda a: a.ctypes.data  # noqa: E731
+    split.dh_can_reach.argtypes = [C.c_void_p, C.POINTER(C.c_float), C.POINTER(C.c_float), C.c_uint32, C.c_uint32, C.c_int]
+    nv, out, visible = C.c_int(0), 0, 0
+    for i in range(len(O)):
+        o, d = _f3(O[i]), _f3(D[i])
+        can = split.dh_can_reach(P(wa.uber), o, d, int(pos[i]), int(size[i]), 128)
+        if not can or i % 4 == 0:
+            v = dh.dh_shadow(P(wa.grid), P(wa.uber), P(wa.bricks), P(boxes), o, d, int(pos[i]), int(size[i]), 0, C.byref(nv))
+            assert can or not v, (i, O[i], D[i], pos[i], size[i])
+            visible += v
+        out += not can
+    return len(O), out, visible
+
+
+def test_rays_out_of_reach_are_occluded(dh, split):  # noqa: F811
+    """Candidate shadow rays of the 1,024-voxel benchmark scene, and the same rays pointed at
+    other emitters and at solid ones of 8 voxels; axis-aligned rays, rays from outside the map
+    and of numbers that are not finite are left to the walk."""
+    hs = ob.HostScene(3)
+    wa = ob.WorldArrays(hs.grid, hs.bricks, hs.lights)
+    O, D, LI = _candidate_shadow_rays(wa, hs.lights, 112, 63, lambda f: hs.camera_path(1, 150 + f, 300), False)
+    pos, size = hs.lights["position"], hs.lights["size"]
+    n, out, visible = _compare_reach(dh, split, wa, O, D, pos[LI], size[LI])
+    assert out > 0.1 * n and visible > 100
+    rng = np.random.default_rng(4)
+    li = rng.integers(0, len(pos), len(O))
+    to = np.stack([pos[li] % 1024, pos[li] // 1048576, (pos[li] // 1024) % 1024], 1).astype(np.float32) + np.float32(0.5)
+    size = np.where(rng.random(len(O)) < 0.3, 8, 1)
+    D2 = to - O
+    D2 = (D2 / np.linalg.norm(D2, axis=1, keepdims=True)).astype(np.float32)
+    D2[::9] = D[::9]                                     # a ray that does not head for its emitter
+    D2[1::50, 0] = 0.0
+    D2[2::50] = np.nan
+    O[3::50] -= 2000.0
+    n, out, _ = _compare_reach(dh, split, wa, O, D2, pos[li], size)
+    assert out > 0.1 * n
+
+
 def _compare_first(dh, split, wa, O, D, stepss):  # noqa: F811
     P = lambda a: a.ctypes.data if a is not None else None  # noqa: E731
     split.dh_trace_first.restype = C.c_uint32
