@@ -59,8 +59,8 @@ __global__ void build_light_table_kernel(const uint4* __restrict__ raw, uint32_t
 }
 
 // Per brick the boxes of its opaque voxels (type nibble 15) and of its non-zero voxels,
-// packed as World::bbox describes, and its opacity mask (World::bmask): one warp per brick,
-// 16 voxels a lane, min / max reductions over the warp, a ballot per mask word.
+// packed as World::bbox describes, and its masks of both (World::bmask, bmask0): one warp per
+// brick, 16 voxels a lane, min / max reductions over the warp, a ballot per mask word.
 __device__ __forceinline__ uint32_t warp_box(bool any, const uint32_t lo[3], const uint32_t hi[3]) {
     const bool anyw = __any_sync(0xffffffffu, any);
     uint32_t box = 0u;
@@ -73,7 +73,7 @@ __device__ __forceinline__ uint32_t warp_box(bool any, const uint32_t lo[3], con
 // (list: the bricks to do, or null for bricks 0 .. n - 1)
 __global__ void build_brick_boxes_kernel(const uint32_t* __restrict__ bricks, const uint32_t* __restrict__ list,
                                          uint32_t n, uint32_t* __restrict__ bbox, uint32_t* __restrict__ bbox0,
-                                         uint32_t* __restrict__ bmask) {
+                                         uint32_t* __restrict__ bmask, uint32_t* __restrict__ bmask0) {
     const size_t item = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (item >= n) return;   // whole warps leave together (blockDim a multiple of 32)
     const size_t brick = list ? (size_t)__ldg(list + item) : item;
@@ -85,8 +85,11 @@ __global__ void build_brick_boxes_kernel(const uint32_t* __restrict__ bricks, co
         const uint32_t v = __ldg(bricks + brick * 512u + e);
         const uint32_t c[3] = {e & 7u, (e >> 3) & 7u, e >> 6};
         const bool opaque = ((v & 0xf000u) >> 12) == 15u;
-        const uint32_t word = __ballot_sync(0xffffffffu, opaque);
-        if (lane == i) bmask[brick * 16u + i] = word;
+        const uint32_t word = __ballot_sync(0xffffffffu, opaque), word0 = __ballot_sync(0xffffffffu, v != 0u);
+        if (lane == i) {
+            bmask[brick * 16u + i] = word;
+            bmask0[brick * 16u + i] = word0;
+        }
         if (opaque) {
             for (int a = 0; a < 3; a++) { lo[a] = min(lo[a], c[a]); hi[a] = max(hi[a], c[a]); }
             any = true;
@@ -284,13 +287,14 @@ __device__ __forceinline__ const ViewDev* tile_pixel(const BatchDev& bd, uint32_
 }
 
 // ---- stage 1: primary rays / G-buffer (renderAlbedo, ris.cl:295-389) --------------------
+template <bool BITS>
 __device__ __forceinline__ bool albedo_px(const World& w, const Frame& k, uint2* __restrict__ vd, uint32_t* __restrict__ seeds,
                                           int x, int y) {
     const uint32_t seed = wang_hash((uint32_t)x * 171u + (uint32_t)y * 1773u + k.R0);
     const float3 D = camera_ray(k, x, y);
     uint32_t side = 0;
     float dist = 0.0f;
-    uint32_t voxel = trace_primary(w, k.E, D, &dist, &side);
+    uint32_t voxel = trace_primary<BITS>(w, k.E, D, &dist, &side);
     float alpha = alphaf(voxel);
     float3 outc = mul(to_rgb(voxel), alpha);
     float total = 0.0f;
@@ -339,7 +343,7 @@ __device__ __forceinline__ void list_pixel(const BatchDev& bd, const ViewDev* V,
 // emitters 3,099 -> 2,103 us.
 // LISTS: the kernel also fills the hit list, in tile order (compact_hits_kernel reads the
 // G-buffer back for it: 333 x 187 271 -> 267 us a frame; at 1080p no difference).
-template <int VARIANT, bool LISTS>
+template <int VARIANT, bool LISTS, bool BITS>
 __global__ void __launch_bounds__(kMaxTileThreads, 4) albedo_kernel(const __grid_constant__ BatchDev bd) {
     uint32_t tile, round = 0;
     while (next_tile(bd, bd.counters + kCtrAlbedo, &tile, round)) {
@@ -350,7 +354,7 @@ __global__ void __launch_bounds__(kMaxTileThreads, 4) albedo_kernel(const __grid
         bool hit = false;
         if (in) {
             const World w = V->w;
-            hit = albedo_px(w, k, V->b.vd[V->cur], V->b.seed, x, y);
+            hit = albedo_px<BITS>(w, k, V->b.vd[V->cur], V->b.seed, x, y);
         }
         if (LISTS) list_pixel(bd, V, VARIANT < 2 ? 0u : (uint32_t)(V - bd.views), (uint32_t)y * (uint32_t)k.W + (uint32_t)x, in, hit);
     }
@@ -404,7 +408,7 @@ __device__ __forceinline__ float4 path_trace_px(const World& w, const Frame& k, 
     const float NdotL = fmaxf(0.0f, (N.x * R.x + N.y * R.y) + N.z * R.z);
     float dist2 = 0.0f;
     uint32_t side2 = 0;
-    const uint32_t voxel2 = trace_first<true, true>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z,
+    const uint32_t voxel2 = trace_first<true, true, false>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z,
                                                     128, &dist2, &side2);
     const float3 sampleL = mul(mul(to_rgb(voxel2), (float)((voxel2 & 0xff0000u) >> 16)), INVPI);
     const float TWOPI = 6.28318530717958647692528f;
@@ -1377,10 +1381,10 @@ void launch_build_light_table(const uint4* raw, uint32_t n, float4* geom, float4
 }
 
 void launch_build_brick_boxes(const uint32_t* bricks, const uint32_t* list, uint32_t n, uint32_t* bbox, uint32_t* bbox0,
-                              uint32_t* bmask, cudaStream_t s) {
+                              uint32_t* bmask, uint32_t* bmask0, cudaStream_t s) {
     const size_t threads = (size_t)n * 32u;
     if (threads)
-        dev::build_brick_boxes_kernel<<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(bricks, list, n, bbox, bbox0, bmask);
+        dev::build_brick_boxes_kernel<<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(bricks, list, n, bbox, bbox0, bmask, bmask0);
 }
 
 void launch_commit_bricks(const uint32_t* list, const uint32_t* voxels, uint32_t n, uint32_t* bricks, cudaStream_t s) {
@@ -1400,15 +1404,22 @@ void launch_path_trace(const BatchDev& bd, cudaStream_t s) {
     launch_tiles(dev::path_trace_kernel, b, kCtrAlbedo, s, K_ALBEDO);
 }
 
+// Views of at most this many pixels walk bricks by the masks of their non-zero voxels: small
+// frames wait for their longest ray, whose brick walk reads a line instead of a sector a row
+// (333 x 187: 42.5 us -> 35.3, 640 x 360: 41.7 -> 36.3, 1280 x 720: 153 -> 144); larger ones are
+// bound by instructions, of which a mask takes more (1080p: 393 -> 405, 3840 x 2160: 2,106 ->
+// 2,176).
+constexpr uint32_t kBitsPixels = 1u << 20;
 void launch_batch_albedo(const BatchDev& bd, int variant, cudaStream_t s) {
+    const bool bits = variant != 2 && bd.totalPixels <= kBitsPixels && bd.one.w.bmask0;
     if (bd.lists) {
         // all of the frame's list lengths and cursors at once
         cudaMemsetAsync(bd.counters, 0, kCounters * sizeof(uint32_t), s);
-        if (variant == 2) launch_tiles(dev::albedo_kernel<2, true>, bd, kCtrAlbedo, s, K_ALBEDO);
-        else launch_tiles(dev::albedo_kernel<0, true>, bd, kCtrAlbedo, s, K_ALBEDO);
+        if (variant == 2) launch_tiles(dev::albedo_kernel<2, true, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        else launch_tiles(bits ? dev::albedo_kernel<0, true, true> : dev::albedo_kernel<0, true, false>, bd, kCtrAlbedo, s, K_ALBEDO);
     } else {
-        if (variant == 2) launch_tiles(dev::albedo_kernel<2, false>, bd, kCtrAlbedo, s, K_ALBEDO);
-        else launch_tiles(dev::albedo_kernel<0, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        if (variant == 2) launch_tiles(dev::albedo_kernel<2, false, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        else launch_tiles(bits ? dev::albedo_kernel<0, false, true> : dev::albedo_kernel<0, false, false>, bd, kCtrAlbedo, s, K_ALBEDO);
     }
 }
 

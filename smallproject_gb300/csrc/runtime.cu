@@ -91,15 +91,16 @@ static int upload(World& w) {
             d.cap = 0;
             CU(cudaMalloc(&d.bricks, (size_t)cap * kBrick * sizeof(uint32_t)), "cudaMalloc(bricks)");
             CU(cudaMalloc(&d.bbox, (size_t)cap * 2u * sizeof(uint32_t)), "cudaMalloc(brick boxes)");
-            CU(cudaMalloc(&d.bmask, (size_t)cap * 16u * sizeof(uint32_t)), "cudaMalloc(brick masks)");
+            CU(cudaMalloc(&d.bmask, (size_t)cap * 32u * sizeof(uint32_t)), "cudaMalloc(brick masks)");
             d.cap = cap;
         }
         d.bbox0 = d.bbox + d.cap;
+        d.bmask0 = d.bmask + (size_t)d.cap * 16u;
         CU(cudaMemcpy(d.grid, w.grid.data(), kGridSize * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload grid");
         if (w.brickHigh)
             CU(cudaMemcpy(d.bricks, w.bricks.data(), (size_t)w.brickHigh * kBrick * sizeof(uint32_t), cudaMemcpyHostToDevice),
                "upload bricks");
-        launch_build_brick_boxes(d.bricks, nullptr, w.brickHigh, d.bbox, d.bbox0, d.bmask, 0);
+        launch_build_brick_boxes(d.bricks, nullptr, w.brickHigh, d.bbox, d.bbox0, d.bmask, d.bmask0, 0);
         sent = w.brickHigh;
     } else if (w.dirtyCount) {
         if (w.dirtyCount > d.stageCap) {
@@ -134,7 +135,7 @@ static int upload(World& w) {
             const size_t bytes = (voxOff + (size_t)k * kBrick) * sizeof(uint32_t);
             CU(cudaMemcpy(d.stageDev, d.stageHost, bytes, cudaMemcpyHostToDevice), "commit bricks");
             launch_commit_bricks(d.stageDev, d.stageDev + voxOff, k, d.bricks, 0);
-            launch_build_brick_boxes(d.bricks, d.stageDev, k, d.bbox, d.bbox0, d.bmask, 0);
+            launch_build_brick_boxes(d.bricks, d.stageDev, k, d.bbox, d.bbox0, d.bmask, d.bmask0, 0);
         }
     }
     if (full || w.gridDirty) {
@@ -219,6 +220,7 @@ vxr::dev::World dev_world(vxr_view* v) {
     w.ucell0 = d.ucell0;
     w.ucell = d.ucell;
     w.bmask = d.bmask;
+    w.bmask0 = d.bmask0;
     w.gbox = d.gbox;
     w.gbox0 = d.gbox0;
     w.lgeom = d.lgeom;

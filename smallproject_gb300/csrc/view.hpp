@@ -20,6 +20,7 @@ struct DeviceWorld {
     uint32_t* bbox = nullptr;        // boxes of the opaque voxels per brick (brick skipping),
     uint32_t* bbox0 = nullptr;       // then those of the non-zero voxels (bbox + cap)
     uint32_t* bmask = nullptr;       // opacity masks per brick (16 words, dev::World::bmask)
+    uint32_t* bmask0 = nullptr;      // masks of the non-zero voxels, the allocation's second half (bmask0)
     uint4* ucell0 = nullptr;         // mask and box of the non-zero cells per uber cell (32^3)
     unsigned long long* ucell = nullptr;   // shadow rays' mask of an uber cell (32^3, dev::World::ucell)
     uint2* gbox = nullptr;           // grid cells with their bricks' boxes (128^3, dev::World::gbox),

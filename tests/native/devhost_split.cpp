@@ -75,16 +75,19 @@ int dh_can_reach(const uint8_t* uber, const float* O, const float* D, uint32_t p
                             size, steps);
 }
 
-// trace_first with a budget, or a primary ray (boxes: gbox0 given)
+// trace_first with a budget, or a primary ray (boxes: gbox0 given; masks of the bricks' non-zero
+// voxels: bmask0 given)
 uint32_t dh_trace_first(const uint32_t* grid, const uint8_t* uber, const uint32_t* bricks, const uint32_t* ucell0, const uint32_t* gbox0,
-                        const float* O, const float* D, int budget, int steps, float* dist, uint32_t* side) {
+                        const uint32_t* bmask0, const float* O, const float* D, int budget, int steps, float* dist, uint32_t* side) {
     World w = make_world(grid, uber, bricks);
     w.ucell0 = reinterpret_cast<const uint4*>(ucell0);
     w.gbox0 = reinterpret_cast<const uint2*>(gbox0);
+    w.bmask0 = bmask0;
     *dist = 0.0f;
     *side = 0;
-    if (!budget) return trace_primary(w, f3(O[0], O[1], O[2]), f3(D[0], D[1], D[2]), dist, side);
-    const auto f = gbox0 ? trace_first<true, true> : trace_first<false, true>;
+    if (!budget)
+        return (bmask0 ? trace_primary<true> : trace_primary<false>)(w, f3(O[0], O[1], O[2]), f3(D[0], D[1], D[2]), dist, side);
+    const auto f = !gbox0 ? trace_first<false, true, false> : bmask0 ? trace_first<true, true, true> : trace_first<true, true, false>;
     return f(w, O[0], O[1], O[2], D[0], D[1], D[2], steps, dist, side);
 }
 

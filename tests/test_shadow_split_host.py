@@ -68,9 +68,10 @@ def uber_cells0(grid, bricks, boxed):
     return np.ascontiguousarray(out.reshape(-1, 4)), gbox
 
 
-def brick_masks(bricks):
-    """World::bmask as the GPU builds it (build_brick_boxes_kernel)."""
-    op = ((bricks.reshape(-1, 16, 32) >> 12) & 15) == 15
+def brick_masks(bricks, nonzero=False):
+    """World::bmask (nonzero: bmask0) as the GPU builds it (build_brick_boxes_kernel)."""
+    v = bricks.reshape(-1, 16, 32)
+    op = v != 0 if nonzero else ((v >> 12) & 15) == 15
     return (op.astype(np.uint32) << np.arange(32, dtype=np.uint32)).sum(axis=2, dtype=np.uint32)
 
 
@@ -190,16 +191,16 @@ def test_rays_out_of_reach_are_occluded(dh, split):  # noqa: F811
 def _compare_first(dh, split, wa, O, D, stepss):  # noqa: F811
     P = lambda a: a.ctypes.data if a is not None else None  # noqa: E731
     split.dh_trace_first.restype = C.c_uint32
-    split.dh_trace_first.argtypes = [C.c_void_p] * 5 + [C.POINTER(C.c_float)] * 2 + [C.c_int, C.c_int, C.POINTER(C.c_float),
+    split.dh_trace_first.argtypes = [C.c_void_p] * 6 + [C.POINTER(C.c_float)] * 2 + [C.c_int, C.c_int, C.POINTER(C.c_float),
                                                                                      C.POINTER(C.c_uint32)]
     hits = 0
-    for boxed in (True, False):
+    for boxed, bits in ((True, None), (False, None), (True, brick_masks(wa.bricks, nonzero=True))):
         uc, gb = uber_cells0(wa.grid, wa.bricks, boxed)
         for i in range(len(O)):
             o, d, steps = _f3(O[i]), _f3(D[i]), int(stepss[i])
             da, sa, db, sb = C.c_float(0), C.c_uint32(0), C.c_float(0), C.c_uint32(0)
             a = dh.dh_trace(0, P(wa.grid), P(wa.uber), P(wa.bricks), o, d, steps, 0, 0, C.byref(da), C.byref(sa))
-            b = split.dh_trace_first(P(wa.grid), P(wa.uber), P(wa.bricks), P(uc), P(gb), o, d, int(steps < 999999), steps, C.byref(db),
+            b = split.dh_trace_first(P(wa.grid), P(wa.uber), P(wa.bricks), P(uc), P(gb), P(bits), o, d, int(steps < 999999), steps, C.byref(db),
                                      C.byref(sb))
             assert (a, sa.value) == (b, sb.value) and \
                 np.float32(da.value).view(np.uint32) == np.float32(db.value).view(np.uint32), (i, O[i], D[i], steps)
