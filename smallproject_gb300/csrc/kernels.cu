@@ -70,7 +70,7 @@ __device__ __forceinline__ uint32_t warp_box(bool any, const uint32_t lo[3], con
     }
     return anyw ? box : kNoOpaque;
 }
-// (list: the bricks to do, or null for bricks 0 .. n - 1)
+// (list: the bricks to do, or null for bricks 0 .. n - 1; bmask and bmask0 may be null)
 __global__ void build_brick_boxes_kernel(const uint32_t* __restrict__ bricks, const uint32_t* __restrict__ list,
                                          uint32_t n, uint32_t* __restrict__ bbox, uint32_t* __restrict__ bbox0,
                                          uint32_t* __restrict__ bmask, uint32_t* __restrict__ bmask0) {
@@ -86,7 +86,7 @@ __global__ void build_brick_boxes_kernel(const uint32_t* __restrict__ bricks, co
         const uint32_t c[3] = {e & 7u, (e >> 3) & 7u, e >> 6};
         const bool opaque = ((v & 0xf000u) >> 12) == 15u;
         const uint32_t word = __ballot_sync(0xffffffffu, opaque), word0 = __ballot_sync(0xffffffffu, v != 0u);
-        if (lane == i) {
+        if (bmask && lane == i) {
             bmask[brick * 16u + i] = word;
             bmask0[brick * 16u + i] = word0;
         }
@@ -143,8 +143,10 @@ __global__ void __launch_bounds__(256) build_cells_kernel(const uint32_t* __rest
     const uint32_t i = ((u & 31u) * 4u + cx) + (((u >> 5) & 31u) * 4u + cz) * 128u + ((u >> 10) * 4u + cy) * 16384u;
     const uint32_t c = __ldg(grid + i);
     const bool brick = c & 1u;
-    if (err && brick && (c >> 1) >= nbricks) atomicOr(err, 16u);
-    const uint32_t box = brick && bbox ? __ldg(bbox + (c >> 1)) : 0u, box0 = brick && bbox0 ? __ldg(bbox0 + (c >> 1)) : 0u;
+    const bool bad = err && brick && (c >> 1) >= nbricks;
+    if (bad) atomicOr(err, 16u);
+    const uint32_t box = brick && bbox && !bad ? __ldg(bbox + (c >> 1)) : 0u,
+                   box0 = brick && bbox0 && !bad ? __ldg(bbox0 + (c >> 1)) : 0u;
     if (out.gbox) out.gbox[i] = make_uint2(c, box);
     if (out.gbox0) out.gbox0[i] = make_uint2(c, box0);
     const bool stops = brick ? box != kNoOpaque : (((c >> 1) & 0xf000u) >> 12) == 15u;
@@ -408,7 +410,7 @@ __device__ __forceinline__ float4 path_trace_px(const World& w, const Frame& k, 
     const float NdotL = fmaxf(0.0f, (N.x * R.x + N.y * R.y) + N.z * R.z);
     float dist2 = 0.0f;
     uint32_t side2 = 0;
-    const uint32_t voxel2 = trace_first<true, true, false>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z,
+    const uint32_t voxel2 = trace_first<1, true, false>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z,
                                                     128, &dist2, &side2);
     const float3 sampleL = mul(mul(to_rgb(voxel2), (float)((voxel2 & 0xff0000u) >> 16)), INVPI);
     const float TWOPI = 6.28318530717958647692528f;
@@ -499,8 +501,9 @@ struct ShadowWarp {
 // the 1080p frame with 65,536 emitters: 1,563 us before, 728 us now (shading's 1,801,412:
 // 1,330 and 623 us); 58,047 rays of a 333 x 187 frame, bound by the longest ray: 77 and 46
 // us. 7 blocks a SM (72 registers): 6 took 768 us, 8 (64 registers, spills) 755 us.
-// MASK: the world has cell boxes and opacity masks (else cells and voxels are read).
-template <int VARIANT, bool MASK, int MINB>
+// BOX: 1 the world has cell boxes and opacity masks, 2 brick boxes only, 0 neither (cells and
+// voxels are read).
+template <int VARIANT, int BOX, int MINB>
 __global__ void __launch_bounds__(128, MINB) shadow_kernel(const __grid_constant__ BatchDev bd, int countIdx, int fetchIdx,
                                                            int planeSel) {
     __shared__ ShadowWarp s_warp[4];
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(128, MINB) shadow_kernel(const __grid_constant
                 const float t = __uint_as_float(rec.x);
                 float d = t * 8.0f;
                 uint32_t side = (rec.y >> 21) & 3u;
-                hit = brick == kSolidCell || brick_task<MASK>(view(owner)->w, brick, rec.y, t, q.out[slot], side, g, &d, &side);
+                hit = brick == kSolidCell || brick_task<BOX == 1>(view(owner)->w, brick, rec.y, t, q.out[slot], side, g, &d, &side);
                 if (hit) atomicMin(&q.first[owner], (uint32_t)(lane << 1) | (visible(owner, d + g.to, side) ? 1u : 0u));
             }
         }
@@ -644,8 +647,9 @@ __global__ void __launch_bounds__(128, MINB) shadow_kernel(const __grid_constant
                     if ((alive >> owner) & 1u) {
                         const World& w = view(owner)->w;
                         const uint32_t i = rec.y & 0x1FFFFFu;
-                        const uint2 o = MASK ? __ldg(w.gbox + i) : make_uint2(__ldg(w.grid + i), 0u);
-                        kind = grid_task<MASK>(o.x, o.y, rec.y, ray(owner), &out);
+                        uint2 o = BOX == 1 ? __ldg(w.gbox + i) : make_uint2(__ldg(w.grid + i), 0u);
+                        if (BOX == 2 && (o.x & 1u)) o.y = __ldg(w.bbox + (o.x >> 1));
+                        kind = grid_task<BOX != 0>(o.x, o.y, rec.y, ray(owner), &out);
                         if (kind == 2) brick = o.x >> 1;
                     }
                 }
@@ -1458,11 +1462,12 @@ static void launch_shadow(const BatchDev& bd, int countIdx, int planeSel, cudaSt
     } else {
         if constexpr (VARIANT == 0) {
             if (!bd.one.w.bmask) {   // a caller's bricks (vxr_render_frame_noalloc): no masks
-                launch_shadow_rays(dev::shadow_kernel<0, false, kShadowMinBlocks>, bd, countIdx, planeSel, s);
+                launch_shadow_rays(bd.one.w.bbox ? dev::shadow_kernel<0, 2, kShadowMinBlocks> : dev::shadow_kernel<0, 0, kShadowMinBlocks>,
+                                   bd, countIdx, planeSel, s);
                 return;
             }
         }
-        launch_shadow_rays(dev::shadow_kernel<VARIANT, true, kShadowMinBlocks>, bd, countIdx, planeSel, s);
+        launch_shadow_rays(dev::shadow_kernel<VARIANT, 1, kShadowMinBlocks>, bd, countIdx, planeSel, s);
     }
 }
 // 64 registers: at 1080p 914 us against 937 (7 blocks a SM), 988 (6) and 987 (5)

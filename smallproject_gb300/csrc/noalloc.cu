@@ -6,8 +6,8 @@
 // vxr_render_frame_noalloc renders one frame for them from device buffers they already
 // own (the world grid, its bricks and the light list) into an image buffer they own.
 // Everything else the frame needs - G-buffer, seeds, both reservoir planes, the hit
-// list, the shadow-ray queue, the 32^3 uber grid, the per-light table, the counters and
-// the device error word - lives in one file-scope
+// list, the shadow-ray queue, the uber cells' tables, the brick boxes of a world of up to
+// 32,768 bricks, the per-light table, the counters and the device error word - lives in one file-scope
 // __device__ array of fixed size, which every GPU that loads this library holds until
 // the process exits (VXR_NOALLOC_SCRATCH_BYTES = 10,518,784 bytes, 10.0 MiB).
 //
@@ -47,6 +47,8 @@ static_assert(kOffSeed % 256 == 0 && kOffCA % 256 == 0 && kOffUber % 256 == 0 &&
                   kOffHits % 256 == 0 && kOffQA % 256 == 0 && kOffErr % 256 == 0,
               "scratch regions must stay 256-byte aligned");
 static_assert(16 * kMaxLights >= (16 + 8) * 32 * 32 * 32, "the uber cells' masks must fit the region of the widened lights");
+// bricks whose boxes (two words each) fit what the uber cells' masks leave of that region
+constexpr size_t kMaxBoxes = (16 * kMaxLights - (16 + 8) * 32 * 32 * 32) / 8;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -125,7 +127,14 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     // table's kernel reads
     uint4* ucell0 = raw;
     unsigned long long* ucell = (unsigned long long*)(ucell0 + 32 * 32 * 32);
-    vxr::launch_build_cells(grid, nullptr, nullptr, s + kOffUber, ucell, ucell0, nullptr, nullptr, nbricks, err, st);
+    // and, behind them, when the world's bricks are few enough, the boxes of their opaque and of
+    // their non-zero voxels. Reading every brick once (3,734 bricks 3 us, 16,122 some 8) pays
+    // for itself: a frame in us without and with boxes, 256 x 144 of 3,734 bricks 255 and 239,
+    // 200 x 120 of 16,122 337 and 330, 160 x 90 of 15,547 with 30,000 emitters 514 and 392.
+    uint32_t* box = nbricks <= kMaxBoxes ? (uint32_t*)(ucell + 32 * 32 * 32) : nullptr;
+    uint32_t* box0 = box ? box + nbricks : nullptr;
+    if (box) vxr::launch_build_brick_boxes(bricks, nullptr, nbricks, box, box0, nullptr, nullptr, st);
+    vxr::launch_build_cells(grid, box, box0, s + kOffUber, ucell, ucell0, nullptr, nullptr, nbricks, err, st);
     CUN(cudaGetLastError(), "world kernels");
     uint32_t herr = 0;
     CUN(cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "read error word");
@@ -136,8 +145,8 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     w.grid = grid;
     w.uber = s + kOffUber;
     w.bricks = bricks;
-    w.bbox = nullptr;   // no room for brick boxes: rays walk every brick they meet
-    w.bbox0 = nullptr;
+    w.bbox = box;   // null: rays walk every brick they meet
+    w.bbox0 = box0;
     w.ubox0 = nullptr;
     w.ucell = ucell;
     w.ucell0 = ucell0;

@@ -87,7 +87,7 @@ uint32_t dh_trace_first(const uint32_t* grid, const uint8_t* uber, const uint32_
     *side = 0;
     if (!budget)
         return (bmask0 ? trace_primary<true> : trace_primary<false>)(w, f3(O[0], O[1], O[2]), f3(D[0], D[1], D[2]), dist, side);
-    const auto f = !gbox0 ? trace_first<false, true, false> : bmask0 ? trace_first<true, true, true> : trace_first<true, true, false>;
+    const auto f = !gbox0 ? trace_first<0, true, false> : bmask0 ? trace_first<1, true, true> : trace_first<1, true, false>;
     return f(w, O[0], O[1], O[2], D[0], D[1], D[2], steps, dist, side);
 }
 
