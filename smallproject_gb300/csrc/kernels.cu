@@ -43,11 +43,14 @@ namespace dev {
 
 __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t code) { atomicOr(err, code); }
 
-// Light centre/emission from the reference records (tools.cl:600-607, phat.cl:8-12).
-__global__ void build_light_table_kernel(const uint4* __restrict__ raw, uint32_t n, float4* geom, float4* emit) {
+// Light centre/emission from the reference records (tools.cl:600-607, phat.cl:8-12): n records
+// of WORDS words, (position, voxel, size) first.
+template <int WORDS>
+__global__ void build_light_table_kernel(const uint32_t* __restrict__ raw, uint32_t n, float4* geom, float4* emit) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint4 l = raw[i];  // (position, voxel, size, 0)
+    const uint32_t* r = raw + (size_t)i * WORDS;
+    const uint4 l = WORDS == 4 ? *reinterpret_cast<const uint4*>(r) : make_uint4(r[0], r[1], r[2], 0u);
     const uint32_t y = l.x / (1024u * 1024u), z = (l.x / 1024u) % 1024u, x = l.x % 1024u;
     const float size = (float)l.z;
     const float half = 0.5f * size;
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__(256) build_cells_kernel(const uint32_t* __rest
     const uint32_t c = __ldg(grid + i);
     const bool brick = c & 1u;
     const bool bad = err && brick && (c >> 1) >= nbricks;
-    if (bad) atomicOr(err, 16u);
+    if (bad) atomicOr(err, kBadGrid);
     const uint32_t box = brick && bbox && !bad ? __ldg(bbox + (c >> 1)) : 0u,
                    box0 = brick && bbox0 && !bad ? __ldg(bbox0 + (c >> 1)) : 0u;
     if (out.gbox) out.gbox[i] = make_uint2(c, box);
@@ -253,6 +256,7 @@ __device__ __forceinline__ void append_ray(const BatchDev& bd, int counter, bool
 // from the queue cursor `ctr` until it is drained; otherwise the launch has one block per
 // tile and the hardware block scheduler balances them. `round` counts calls (starts at 0).
 __device__ __forceinline__ bool next_tile(const BatchDev& bd, uint32_t* ctr, uint32_t* tile, uint32_t& round) {
+    if (bd.halt && (*bd.halt & kBadGrid)) return false;
     if (!bd.persistent) {
         *tile = blockIdx.x;
         return round++ == 0;
@@ -1379,9 +1383,10 @@ BatchDev single_batch(const dev::World& w, const dev::Frame& k, const ViewBuffer
     return bd;
 }
 
-void launch_build_light_table(const uint4* raw, uint32_t n, float4* geom, float4* emit, cudaStream_t s) {
-    if (n == 0) return;
-    dev::build_light_table_kernel<<<(n + 255) / 256, 256, 0, s>>>(raw, n, geom, emit);
+void launch_build_light_table(const uint32_t* raw, int words, uint32_t n, float4* geom, float4* emit, cudaStream_t s) {
+    const unsigned nb = (n + 255u) / 256u;
+    if (n && words == 4) dev::build_light_table_kernel<4><<<nb, 256, 0, s>>>(raw, n, geom, emit);
+    else if (n) dev::build_light_table_kernel<3><<<nb, 256, 0, s>>>(raw, n, geom, emit);
 }
 
 void launch_build_brick_boxes(const uint32_t* bricks, const uint32_t* list, uint32_t n, uint32_t* bbox, uint32_t* bbox0,

@@ -79,6 +79,8 @@ struct KernelTimer {
 // of at most 2^27 pixels each.
 constexpr uint32_t kMaxBatchViews = 16;
 constexpr int kMaxTileThreads = 256;      // threads of a pixel-stage block (tile_x * tile_y)
+constexpr uint32_t kBadGrid = 16u;        // error flag: a grid cell points past the bricks
+
 struct BatchDev {
     ViewDev one;
     const ViewDev* views = nullptr;       // device table when nviews > 1
@@ -106,6 +108,7 @@ struct BatchDev {
     float4* qA = nullptr;                 // shadow-ray requests: (origin, bits(entry))
     float4* qB = nullptr;                 //                      (direction, bits(light))
     uint32_t* counters = nullptr;         // kCounters words
+    const uint32_t* halt = nullptr;       // the pixel stages do nothing when this word has kBadGrid (null: not asked)
     KernelTimer* timer = nullptr;         // host object (never dereferenced on the device)
 };
 
@@ -123,7 +126,8 @@ struct Tuning {
 };
 
 size_t brick_cache_smem(int log2);   // shared memory of the shadow tracer's brick-cache variant
-void launch_build_light_table(const uint4* raw, uint32_t n, float4* geom, float4* emit, cudaStream_t s);
+// words: 4 (raw 16-byte aligned) or 3, those of a record
+void launch_build_light_table(const uint32_t* raw, int words, uint32_t n, float4* geom, float4* emit, cudaStream_t s);
 void launch_build_brick_boxes(const uint32_t* bricks, const uint32_t* list, uint32_t n, uint32_t* bbox, uint32_t* bbox0,
                               uint32_t* bmask, uint32_t* bmask0, cudaStream_t s);
 void launch_commit_bricks(const uint32_t* list, const uint32_t* voxels, uint32_t n, uint32_t* bricks, cudaStream_t s);

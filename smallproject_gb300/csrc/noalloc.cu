@@ -36,8 +36,8 @@ constexpr size_t kOffHB = kOffHA + 16 * kMaxPx;                // float4 [kMaxPx
 constexpr size_t kOffUber = kOffHB + 16 * kMaxPx;              // uint8 [32^3]
 constexpr size_t kOffGeom = kOffUber + 32 * 32 * 32;           // float4 [kMaxLights]
 constexpr size_t kOffEmit = kOffGeom + 16 * kMaxLights;        // float4 [kMaxLights]
-constexpr size_t kOffRaw = kOffEmit + 16 * kMaxLights;         // uint4 [kMaxLights]
-constexpr size_t kOffHits = kOffRaw + 16 * kMaxLights;         // uint32 [kMaxPx] hit list
+constexpr size_t kOffTables = kOffEmit + 16 * kMaxLights;      // 16 * kMaxLights bytes: the uber cells' tables, brick boxes
+constexpr size_t kOffHits = kOffTables + 16 * kMaxLights;      // uint32 [kMaxPx] hit list
 constexpr size_t kOffQA = kOffHits + 4 * kMaxPx;               // float4 [kMaxPx] shadow requests
 constexpr size_t kOffQB = kOffQA + 16 * kMaxPx;                // float4 [kMaxPx]
 constexpr size_t kOffErr = kOffQB + 16 * kMaxPx;               // uint32 error word, then the work-list counters
@@ -46,8 +46,8 @@ static_assert(kScratchBytes == VXR_NOALLOC_SCRATCH_BYTES, "scratch size must mat
 static_assert(kOffSeed % 256 == 0 && kOffCA % 256 == 0 && kOffUber % 256 == 0 && kOffGeom % 256 == 0 &&
                   kOffHits % 256 == 0 && kOffQA % 256 == 0 && kOffErr % 256 == 0,
               "scratch regions must stay 256-byte aligned");
-static_assert(16 * kMaxLights >= (16 + 8) * 32 * 32 * 32, "the uber cells' masks must fit the region of the widened lights");
-// bricks whose boxes (two words each) fit what the uber cells' masks leave of that region
+static_assert(16 * kMaxLights >= (16 + 8) * 32 * 32 * 32, "the uber cells' tables must fit their region");
+// bricks whose boxes (two words each) fit what they leave of it
 constexpr size_t kMaxBoxes = (16 * kMaxLights - (16 + 8) * 32 * 32 * 32) / 8;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -74,12 +74,6 @@ int scratch_for_current_device(unsigned char** out) {
     }
     *out = g_scratch_ptr[dev];
     return VXR_OK;
-}
-
-// vxr_light (12 bytes) -> the 16-byte records the light-table kernel reads
-__global__ void widen_lights_kernel(const vxr_light* __restrict__ in, uint32_t n, uint4* out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = make_uint4(in[i].position, in[i].voxel, in[i].size, 0u);
 }
 
 }  // namespace
@@ -115,17 +109,14 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     CUN(cudaMemsetAsync(err, 0, sizeof(uint32_t), st), "clear error word");
 
     // derive the light table and the uber cells' tables in scratch; the latter's kernel also
-    // validates the grid, before any traversal reads the bricks through it
-    uint4* raw = (uint4*)(s + kOffRaw);
+    // checks the grid and raises kBadGrid, which keeps the pixel stages from reading bricks
+    // through a bad one and from writing the image: one wait, at the end (with a wait for the
+    // check in between, and light records widened by a kernel of their own, 239 us)
     float4* geom = (float4*)(s + kOffGeom);
     float4* emit = (float4*)(s + kOffEmit);
-    if (nlights) {
-        widen_lights_kernel<<<(nlights + 255) / 256, 256, 0, st>>>(lights, nlights, raw);
-        vxr::launch_build_light_table(raw, nlights, geom, emit, st);
-    }
-    // the uber cells' masks take the place of the widened lights, which only the light
-    // table's kernel reads
-    uint4* ucell0 = raw;
+    static_assert(sizeof(vxr_light) == 12, "three words a light");
+    vxr::launch_build_light_table(reinterpret_cast<const uint32_t*>(lights), 3, nlights, geom, emit, st);
+    uint4* ucell0 = (uint4*)(s + kOffTables);
     unsigned long long* ucell = (unsigned long long*)(ucell0 + 32 * 32 * 32);
     // and, behind them, when the world's bricks are few enough, the boxes of their opaque and of
     // their non-zero voxels. Reading every brick once (3,734 bricks 3 us, 16,122 some 8) pays
@@ -136,10 +127,6 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     if (box) vxr::launch_build_brick_boxes(bricks, nullptr, nbricks, box, box0, nullptr, nullptr, st);
     vxr::launch_build_cells(grid, box, box0, s + kOffUber, ucell, ucell0, nullptr, nullptr, nbricks, err, st);
     CUN(cudaGetLastError(), "world kernels");
-    uint32_t herr = 0;
-    CUN(cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "read error word");
-    CUN(cudaStreamSynchronize(st), "grid check");
-    if (herr & 16u) return vxr::set_error(VXR_E_INVALID, "vxr_render_frame_noalloc: grid references a brick >= nbricks");
 
     vxr::dev::World w;
     w.grid = grid;
@@ -181,14 +168,18 @@ extern "C" int vxr_render_frame_noalloc(const uint32_t* grid, const uint32_t* br
     const vxr::Tuning sh;
     vxr::BatchDev bd = vxr::single_batch(w, f, b, 0, point, sh);
     bd.lists = 1;
+    bd.halt = err;
     const int variant = point ? 1 : 0;
     vxr::launch_batch_albedo(bd, variant, st);
     vxr::launch_batch_candidates(bd, variant, nullptr, st);
     vxr::launch_batch_spatial(bd, variant, st);
     vxr::launch_batch_shade(bd, variant, st);
     CUN(cudaGetLastError(), "stage kernels");
+    uint32_t herr = 0;
     CUN(cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "read error word");
     CUN(cudaStreamSynchronize(st), "vxr_render_frame_noalloc");
+    if (herr & vxr::kBadGrid)
+        return vxr::set_error(VXR_E_INVALID, "vxr_render_frame_noalloc: grid references a brick >= nbricks");
     if (herr) return vxr::set_error(VXR_E_DEVICE, "vxr_render_frame_noalloc: " + vxr::device_flags_message(herr));
     return VXR_OK;
 }

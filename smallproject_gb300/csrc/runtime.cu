@@ -171,7 +171,7 @@ static int upload(World& w) {
         std::vector<uint4> raw(need, make_uint4(0, 0, 1, 0));
         for (uint32_t i = 0; i < nl; i++) raw[i] = make_uint4(w.lights[i].position, w.lights[i].voxel, w.lights[i].size, 0);
         CU(cudaMemcpy(d.lraw, raw.data(), need * sizeof(uint4), cudaMemcpyHostToDevice), "upload lights");
-        launch_build_light_table(d.lraw, (uint32_t)need, d.lgeom, d.lemit, 0);
+        launch_build_light_table(reinterpret_cast<const uint32_t*>(d.lraw), 4, (uint32_t)need, d.lgeom, d.lemit, 0);
         d.nl = nl;
     }
     CU(cudaGetLastError(), "world kernels launch");
