@@ -301,7 +301,7 @@ __device__ __forceinline__ const ViewDev* tile_pixel(const BatchDev& bd, uint32_
 
 // ---- stage 1: primary rays / G-buffer (renderAlbedo, ris.cl:295-389) --------------------
 template <bool BITS>
-__device__ __forceinline__ bool albedo_px(const World& w, const Frame& k, uint2* __restrict__ vd, uint32_t* __restrict__ seeds,
+__device__ __forceinline__ uint32_t albedo_px(const World& w, const Frame& k, uint2* __restrict__ vd, uint32_t* __restrict__ seeds,
                                           int x, int y) {
     const uint32_t seed = wang_hash((uint32_t)x * 171u + (uint32_t)y * 1773u + k.R0);
     const float3 D = camera_ray(k, x, y);
@@ -334,15 +334,47 @@ __device__ __forceinline__ bool albedo_px(const World& w, const Frame& k, uint2*
     const size_t i = (size_t)y * k.W + x;
     vd[i] = make_uint2(enc | (side << 24), __float_as_uint(total));
     seeds[i] = seed;
-    return (enc & 0x00FFFFFFu) != 0u;
+    return (enc & 0x00FFFFFFu) != 0u ? min(side, 2u) : 3u;
 }
 
-// Where pixel i of the view (number v of its batch) goes after its primary ray: a hit pixel to
-// the hit list, the others get the empty reservoir (ris.cl:34,123). Every thread of a block
-// calls it together.
-__device__ __forceinline__ void list_pixel(const BatchDev& bd, const ViewDev* V, uint32_t v, uint32_t i, bool in, bool hit) {
-    const uint32_t slot = block_append(bd.counters + kCtrHits, hit);
-    if (hit) {
+// block_append of three groups, one after the other: group 0, 1 or 2, or 3 for no slot. (Blocks
+// of whole warps, at most kMaxTileThreads: the first warp adds the warps' counts up.)
+static_assert(kMaxTileThreads <= 256, "8 warps a group");
+__device__ __forceinline__ uint32_t block_append_grouped(uint32_t* counter, uint32_t group) {
+    __shared__ uint32_t s_first[32];   // 8 group + warp: the warp's count, then its first slot
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    uint32_t rank = 0;
+    for (uint32_t g = 0; g < 3; g++) {
+        const unsigned m = __ballot_sync(0xffffffffu, group == g);
+        if (group == g) rank = (uint32_t)__popc(m & ((1u << lane) - 1u));
+        if (lane == g) s_first[8u * g + warp] = (uint32_t)__popc(m);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t c = lane < 24u && (lane & 7u) < (blockDim.x >> 5) ? s_first[lane] : 0u;
+        uint32_t sum = c;
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= d) sum += o;
+        }
+        uint32_t first = 0;
+        if (lane == 31u && sum) first = atomicAdd(counter, sum);
+        s_first[lane] = __shfl_sync(0xffffffffu, first, 31) + sum - c;
+    }
+    __syncthreads();
+    const uint32_t slot = s_first[8u * min(group, 2u) + warp] + rank;
+    __syncthreads();   // the shared words are reused by the next call
+    return slot;
+}
+
+// Where pixel i of the view (number v of its batch) goes after its primary ray: a pixel that hit
+// a face of axis `face` to the hit list, the others (3) get the empty reservoir (ris.cl:34,123).
+// A block's hits are listed axis by axis, so that most warps of the candidate pass have
+// pixels of one face, where that pays (GROUPED: bd.grouped). Every thread of a block calls it together.
+template <bool GROUPED>
+__device__ __forceinline__ void list_pixel(const BatchDev& bd, const ViewDev* V, uint32_t v, uint32_t i, bool in, uint32_t face) {
+    const uint32_t slot = GROUPED ? block_append_grouped(bd.counters + kCtrHits, face) : block_append(bd.counters + kCtrHits, face < 3u);
+    if (face < 3u) {
         bd.hits[slot] = (v << 27) | i;
     } else if (in) {
         V->b.cA[i] = make_uint4(0u, 6u << 29, 0u, 0u);
@@ -354,9 +386,9 @@ __device__ __forceinline__ void list_pixel(const BatchDev& bd, const ViewDev* V,
 // 3 (1080p: 413 us against 446) and 5 (455). trace_first's cell masks and packed cells, these
 // blocks and compact warps: 1080p, 65,536 emitters 544 -> 393 us, 3840 x 2160 with 1,048,576
 // emitters 3,099 -> 2,103 us.
-// LISTS: the kernel also fills the hit list, in tile order (compact_hits_kernel reads the
-// G-buffer back for it: 333 x 187 271 -> 267 us a frame; at 1080p no difference).
-template <int VARIANT, bool LISTS, bool BITS>
+// LISTS: the kernel also fills the hit list (2: grouped), in tile order (compact_hits_kernel
+// reads the G-buffer back for it: 333 x 187 271 -> 267 us a frame; at 1080p no difference).
+template <int VARIANT, int LISTS, bool BITS>
 __global__ void __launch_bounds__(kMaxTileThreads, 4) albedo_kernel(const __grid_constant__ BatchDev bd) {
     follow_previous();
     uint32_t tile, round = 0;
@@ -365,12 +397,12 @@ __global__ void __launch_bounds__(kMaxTileThreads, 4) albedo_kernel(const __grid
         const ViewDev* V = tile_pixel<VARIANT, true>(bd, tile, &x, &y);
         const Frame& k = V->k;
         const bool in = x < k.W && y < k.H;
-        bool hit = false;
+        uint32_t face = 3u;
         if (in) {
             const World w = V->w;
-            hit = albedo_px<BITS>(w, k, V->b.vd[V->cur], V->b.seed, x, y);
+            face = albedo_px<BITS>(w, k, V->b.vd[V->cur], V->b.seed, x, y);
         }
-        if (LISTS) list_pixel(bd, V, VARIANT < 2 ? 0u : (uint32_t)(V - bd.views), (uint32_t)y * (uint32_t)k.W + (uint32_t)x, in, hit);
+        if (LISTS) list_pixel<LISTS == 2>(bd, V, VARIANT < 2 ? 0u : (uint32_t)(V - bd.views), (uint32_t)y * (uint32_t)k.W + (uint32_t)x, in, face);
     }
 }
 
@@ -443,7 +475,7 @@ __global__ void __launch_bounds__(kMaxTileThreads, 4) path_trace_kernel(const __
 
 // Hit list of the frame over every view (blockIdx.y = view), for frames run stage by stage
 // (whole frames fill it in the primary rays' kernel).
-template <int VARIANT>
+template <int VARIANT, bool GROUPED>
 __global__ void __launch_bounds__(256) compact_hits_kernel(const __grid_constant__ BatchDev bd) {
     const ViewDev* V = view_of<VARIANT>(bd, blockIdx.y);
     const uint32_t n = (uint32_t)V->k.W * (uint32_t)V->k.H;
@@ -452,7 +484,8 @@ __global__ void __launch_bounds__(256) compact_hits_kernel(const __grid_constant
     for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
         const uint32_t i = i0 + threadIdx.x;
         const bool in = i < n;
-        list_pixel(bd, V, blockIdx.y, i, in, in && (vd[i].x & 0x00FFFFFFu) != 0u);
+        const uint32_t word = in ? vd[i].x : 0u;
+        list_pixel<GROUPED>(bd, V, blockIdx.y, i, in, (word & 0x00FFFFFFu) != 0u ? min(word >> 24, 2u) : 3u);
     }
 }
 
@@ -806,8 +839,22 @@ __global__ void __launch_bounds__(CACHE ? 512 : 128, CACHE ? 1 : MINB) shadow_wa
 // pixels x 32 candidates from 1,563 to 914 us, x 4 learned ones from 281 to 166 us.
 // LEARNED: the light index and its source pdf p come from the learned proposal (drawn
 // by the inference kernel) instead of GenerateLightCandidate's uniform 1 / N.
-template <bool POINT, bool LEARNED>
-__device__ __forceinline__ Res ris_reservoir(const ViewDev* V, uint32_t i, uint32_t j, float3* origin) {
+//
+// Emitters behind the shading point's surface have weight 0: such a candidate only counts and
+// draws. Where they are many, a lane first scans its candidates, leaping over the 14 draws that
+// follow the light's, and keeps the random states of those in front; then it works those out
+// one after the other, so that a warp takes as many rounds as its lane with the most of them.
+// A scanned candidate costs a sixth of a worked-out one, so a warp scans on only when a third
+// of its lanes' first two candidates lie behind. SCAN: views that scan (kReachEmitters).
+constexpr uint32_t kScanMin = 16, kScanMax = 32;   // candidates of a pixel (more: no room)
+struct FrontScan {
+    uint32_t jump[128];               // xs_jump(14)
+    uint32_t state[kScanMax][128];    // per thread
+};
+__device__ const XsJump kJump14 = xs_jump(14);
+
+template <bool POINT, bool LEARNED, bool SCAN>
+__device__ __forceinline__ Res ris_reservoir(const ViewDev* V, uint32_t i, uint32_t j, FrontScan* scan, float3* origin) {
     const World w = V->w;
     const Frame& k = V->k;
     const int x = (int)(i % (uint32_t)k.W), y = (int)(i / (uint32_t)k.W);
@@ -828,9 +875,34 @@ __device__ __forceinline__ Res ris_reservoir(const ViewDev* V, uint32_t i, uint3
     // are the rounding of the same real number)
     const bool pow2 = !LEARNED && (nL & (nL - 1u)) == 0u;
     const float nLf = (float)nL;
-    for (uint32_t c = 0; c < k.ncand; c++) {
+    uint32_t count = k.ncand, end = 0;
+    bool front = false;
+    if (SCAN && !POINT && !LEARNED && count >= kScanMin && count <= kScanMax) {
+        const float at = side == 0 ? sp.x : (side == 1 ? sp.y : sp.z);
+        uint32_t s = seed, n = 0;
+        for (uint32_t c = 0; c < k.ncand; c++) {
+            scan->state[n][threadIdx.x] = s;
+            const int li = min(max(f2i(rnd(s) * nLf), 0), (int)nL - 1);
+            const float4 lg = __ldg(w.lgeom + li);
+            // (the sampled point's rounding is below 0.001)
+            const float to = nsign * ((side == 0 ? lg.x : (side == 1 ? lg.y : lg.z)) - at) + 0.5f * lg.w;
+            if (!(to < -0.01f && lg.w <= 1024.0f)) n++;
+            s = xs_leap(scan->jump, s);
+            if (c == 1) {
+                const unsigned m = __activemask();
+                if (3u * __reduce_add_sync(m, n) > 4u * (uint32_t)__popc(m)) break;
+                front = true;
+            }
+        }
+        if (front) {
+            count = n;
+            end = s;
+        }
+    }
+    for (uint32_t c = 0; c < count; c++) {
         int li;
         float p = puni;
+        if (front) seed = scan->state[c][threadIdx.x];
         if (LEARNED) {
             const uint2 cq = __ldg(V->ll.cand + (size_t)c * V->ll.stride + j);
             li = (int)cq.x;
@@ -865,6 +937,10 @@ __device__ __forceinline__ Res ris_reservoir(const ViewDev* V, uint32_t i, uint3
         }
         res_update(res, pow2 ? ph * nLf : ph / p, ph, (uint32_t)li, rnd(seed), pos, inv, nc);
     }
+    if (front) {
+        seed = end;
+        res.M = k.ncand;
+    }
     V->b.seed[i] = seed;
     *origin = spo;
     return res;
@@ -873,7 +949,7 @@ __device__ __forceinline__ Res ris_reservoir(const ViewDev* V, uint32_t i, uint3
 template <bool POINT, bool LEARNED>
 __device__ __forceinline__ void ris_item(const BatchDev& bd, const ViewDev* V, uint32_t e, uint32_t i, uint32_t j) {
     float3 o;
-    const Res res = ris_reservoir<POINT, LEARNED>(V, i, j, &o);
+    const Res res = ris_reservoir<POINT, LEARNED, false>(V, i, j, nullptr, &o);
     if (res.sumW > 0.0f) {   // (no candidates: sumW is 0)
         const float3 L = normalize3(sub(res.pos, o));
         const uint32_t slot = append_slot(bd.counters + kCtrQ1);
@@ -898,6 +974,13 @@ __global__ void __launch_bounds__(128, MINB) ris_kernel(const __grid_constant__ 
 // The same with no request for a ray that cannot reach its emitter.
 template <int VARIANT, bool LEARNED, int MINB>
 __global__ void __launch_bounds__(128, MINB) ris_reach_kernel(const __grid_constant__ BatchDev bd) {
+    FrontScan* scan = nullptr;
+    if constexpr (VARIANT != 1 && !LEARNED) {
+        __shared__ FrontScan s_scan;
+        s_scan.jump[threadIdx.x] = kJump14.w[threadIdx.x];   // 128 threads
+        __syncthreads();
+        scan = &s_scan;
+    }
     follow_previous();
     const uint32_t nh = bd.counters[kCtrHits];
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -911,7 +994,8 @@ __global__ void __launch_bounds__(128, MINB) ris_reach_kernel(const __grid_const
         e = bd.hits[j];
         V = view_of<VARIANT>(bd, e >> 27);
         i = pix_of<VARIANT>(e);
-        res = point_of<VARIANT>(V) ? ris_reservoir<true, LEARNED>(V, i, j, &o) : ris_reservoir<false, LEARNED>(V, i, j, &o);
+        res = point_of<VARIANT>(V) ? ris_reservoir<true, LEARNED, true>(V, i, j, scan, &o)
+                                   : ris_reservoir<false, LEARNED, true>(V, i, j, scan, &o);
     }
     // the warp's requests together: lanes that appended as they came out of the walk would pay
     // an atomic each (learned, 4 candidates: 354 us against 253)
@@ -1402,6 +1486,20 @@ void apply_tuning(BatchDev& bd, const Tuning& tu) {
     bd.earlyOut = tu.earlyOut;
 }
 
+// Rays are tested for their reach when the emitters are at least as many as the map's uber
+// cells: walks then cross few empty ones, and the budget runs out. Candidates and their rays,
+// us without and with the test: 65,536 emitters at 1080p 914 + 728 and 1,001 + 521, learned
+// 166 + 738 and 253 + 415; 1,048,576 at 4K 3,568 + 2,330 and 3,892 + 1,108. Worlds with fewer
+// lose: 4,096 emitters at 720p 417 + 320 and 460 + 280, 1,024 in a 512^3 world 411 + 266 and
+// 435 + 266. Single views only: a batch's views share a launch.
+// The area-light candidates of these views are also scanned for those in front of the surface
+// (FrontScan), and their hits listed by the axis of their face: at 4K, where 63 % of the
+// candidates lie behind, 3,902 us -> 3,061 (3,592 with hits in tile order, as neighbouring
+// pixels see different faces), at 1080p, where 21 % do, 1,003 -> 1,005. In worlds of fewer
+// emitters, whose light tables L1 holds, the scan's shared memory takes that place: 4,096
+// emitters at 720p 418 -> 439 us, 1,024 412 -> 429; and listing by axis costs a small frame
+// 1 % (333 x 187: 211.9 -> 213.2 us).
+constexpr uint32_t kReachEmitters = 32768;
 BatchDev single_batch(const dev::World& w, const dev::Frame& k, const ViewBuffers& b, int cur, bool point, const Tuning& tu) {
     BatchDev bd;
     bd.one.w = w;
@@ -1416,6 +1514,8 @@ BatchDev single_batch(const dev::World& w, const dev::Frame& k, const ViewBuffer
     bd.totalPixels = (uint32_t)k.W * (uint32_t)k.H;
     bd.totalTiles = bd.one.tilesX * (uint32_t)((k.H + tu.by - 1) / tu.by);
     apply_tuning(bd, tu);
+    bd.grouped = !point && k.nlights >= kReachEmitters && k.ncand >= dev::kScanMin && k.ncand <= dev::kScanMax &&
+                 tu.bx * tu.by % 32 == 0;   // (block_append_grouped needs whole warps)
     bd.hits = b.hits;
     bd.qA = b.qA;
     bd.qB = b.qB;
@@ -1465,11 +1565,12 @@ void launch_batch_albedo(const BatchDev& bd, int variant, cudaStream_t s) {
     if (bd.lists) {
         // all of the frame's list lengths and cursors at once
         if (!bd.cleared) cudaMemsetAsync(bd.counters, 0, kCounters * sizeof(uint32_t), s);
-        if (variant == 2) launch_tiles(dev::albedo_kernel<2, true, false>, bd, kCtrAlbedo, s, K_ALBEDO);
-        else launch_tiles(bits ? dev::albedo_kernel<0, true, true> : dev::albedo_kernel<0, true, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        if (variant == 2) launch_tiles(dev::albedo_kernel<2, 1, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        else if (bd.grouped) launch_tiles(bits ? dev::albedo_kernel<0, 2, true> : dev::albedo_kernel<0, 2, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        else launch_tiles(bits ? dev::albedo_kernel<0, 1, true> : dev::albedo_kernel<0, 1, false>, bd, kCtrAlbedo, s, K_ALBEDO);
     } else {
-        if (variant == 2) launch_tiles(dev::albedo_kernel<2, false, false>, bd, kCtrAlbedo, s, K_ALBEDO);
-        else launch_tiles(bits ? dev::albedo_kernel<0, false, true> : dev::albedo_kernel<0, false, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        if (variant == 2) launch_tiles(dev::albedo_kernel<2, 0, false>, bd, kCtrAlbedo, s, K_ALBEDO);
+        else launch_tiles(bits ? dev::albedo_kernel<0, 0, true> : dev::albedo_kernel<0, 0, false>, bd, kCtrAlbedo, s, K_ALBEDO);
     }
 }
 
@@ -1521,13 +1622,6 @@ constexpr int kRisMinBlocks = 8;
 // A block per 128 pixels of the batch, those past the hit list's end leaving at once: a warp's
 // candidates take long enough that the block scheduler balances them better than resident
 // blocks striding over the list (1080p, 7 blocks a SM: 937 us against 1,005).
-// Rays are tested for their reach when the emitters are at least as many as the map's uber
-// cells: walks then cross few empty ones, and the budget runs out. Candidates and their rays,
-// us without and with the test: 65,536 emitters at 1080p 914 + 728 and 1,001 + 521, learned
-// 166 + 738 and 253 + 415; 1,048,576 at 4K 3,568 + 2,330 and 3,892 + 1,108. Worlds with fewer
-// lose: 4,096 emitters at 720p 417 + 320 and 460 + 280, 1,024 in a 512^3 world 411 + 266 and
-// 435 + 266. Single views only: a batch's views share a launch.
-constexpr uint32_t kReachEmitters = 32768;
 template <int VARIANT, bool LEARNED>
 static void launch_ris(const BatchDev& bd, cudaStream_t s) {
     const unsigned nb = (unsigned)(((size_t)bd.totalPixels + 127) / 128);
@@ -1549,7 +1643,9 @@ static void candidates_v(const BatchDev& bd, const LearnedHook* learned, cudaStr
         cudaMemsetAsync(bd.counters + kCtrHits, 0, 4 * sizeof(uint32_t), s);   // hits, q1 requests, q1 fetch, decided rays
         const uint32_t maxPx = VARIANT < 2 ? bd.totalPixels : (uint32_t)(n / bd.nviews + 1);
         Timed tm(bd, K_COMPACT, s);
-        dev::compact_hits_kernel<VARIANT><<<dim3(list_blocks(maxPx, 256, 8), bd.nviews), 256, 0, s>>>(bd);
+        const dim3 nb(list_blocks(maxPx, 256, 8), bd.nviews);
+        if (VARIANT < 2 && bd.grouped) dev::compact_hits_kernel<VARIANT < 2 ? 0 : 2, true><<<nb, 256, 0, s>>>(bd);
+        else dev::compact_hits_kernel<VARIANT < 2 ? 0 : 2, false><<<nb, 256, 0, s>>>(bd);
     }
     const unsigned nb = list_blocks(n, 128, bd.listPerSm);
     bool learnedDone = false;

@@ -754,6 +754,7 @@ static int run_stage(vxr_view* v, int stage, bool fuse, cudaStream_t s, cudaStre
     bd.fuse = fuse ? 1 : 0;
     bd.timer = v->ktimerOn ? v->ktimer : nullptr;
     bd.lists = fuse && !bd.timer ? 1 : 0;
+    if (v->useProposal) bd.grouped = 0;   // its candidates are not scanned
     if (sh.brickCache > 0) {
         if (v->bc.calibrating) {
             bd.bcCount = v->bc.count;
