@@ -297,8 +297,8 @@ KERNEL_PASS_FRAMES = 30   # frames of the per-kernel timing pass (each waited fo
 NFR = 300
 # DRAM bytes per launch of the dominant kernel from the ncu capture of the 960x540 case
 # (profiles/), scaled by 4 to 1920x1080 (the ray count grows with the pixel count)
-NCU_TRAFFIC_1080P = {"shadow_candidates": 4 * (71.57e6 + 2.96e6), "shadow_shading": 4 * (62.44e6 + 1.91e6),
-                     "ris_candidates": 4 * (10.33e6 + 0.01e6), "albedo": 4 * (33.93e6 + 0.47e6)}
+NCU_TRAFFIC_1080P = {"shadow_candidates": 4 * (20.84e6 + 0.00e6), "shadow_shading": 4 * (23.44e6 + 0.00e6),
+                     "ris_candidates": 4 * (10.37e6 + 0.06e6), "albedo": 4 * (14.66e6 + 2.41e6)}
 
 
 def boot_ci(groups, stat, n=2000, seed=0):

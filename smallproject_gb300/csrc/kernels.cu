@@ -543,8 +543,8 @@ struct ShadowWarp {
 // a walker that also steps through bricks keeps 9 of 32 threads busy per instruction, since
 // some lane is always in a brick; with the bricks taken out of the walk and packed densely
 // 18 are, and a ray costs 387 warp instructions instead of 860. 1,894,052 candidate rays of
-// the 1080p frame with 65,536 emitters: 1,563 us before, 728 us now (shading's 1,801,412:
-// 1,330 and 623 us); 58,047 rays of a 333 x 187 frame, bound by the longest ray: 77 and 46
+// the 1080p frame with 65,536 emitters: 1,563 us before, 728 us now, 515 for the three quarters
+// of them in reach (shading's 1,801,412: 1,330 and 616 us); 58,047 rays of a 333 x 187 frame, bound by the longest ray: 77 and 45
 // us. 7 blocks a SM (72 registers): 6 took 768 us, 8 (64 registers, spills) 755 us.
 // BOX: 1 the world has cell boxes and opacity masks, 2 brick boxes only, 0 neither (cells and
 // voxels are read).
@@ -1442,8 +1442,7 @@ struct Timed {
 // A kernel whose launch is made ready while the kernel before it in the stream still runs
 // (programmatic stream serialization; follow_previous is what keeps the order). Frames, us,
 // without and with it: 256 x 144 without allocation 222 and 203, 333 x 187 217 and 212, 640 x 360
-// 329 and 325;
-// large ones do not change. Its blocks are not placed before the others' are done
+// 329 and 325; large ones do not change. Its blocks are not placed before the others' are done
 // (griddepcontrol.launch_dependents at the kernels' start): they would hold places that the
 // blocks still to come then share unevenly (241, 230 and 326 us).
 template <class... P, class... A>
