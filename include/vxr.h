@@ -498,7 +498,8 @@ int vxr_view_error(vxr_view* img, int which, vxr_view* ref, double* mse, double*
 typedef struct vxr_tuning {
     uint32_t tile_x, tile_y;       /* threads of a pixel-stage block; tile_x * tile_y a multiple of 32, <= 256 */
     uint32_t persistent;           /* pixel stages: 1 = resident blocks pull tiles from a queue, 0 = one block per tile */
-    uint32_t shadow_refill;        /* shadow tracer: idle lanes of a warp (1..32) that trigger a refill from the queue */
+    uint32_t shadow_refill;        /* shadow tracer: idle lanes of a warp (1..32) that trigger a refill from the queue (half as
+                                    * many in the candidate pass, a quarter in shading's, at least one) */
     uint32_t shadow_burst;         /* shadow tracer: grid-cell visits per lane between refill checks (1..64, in steps of 4) */
     uint32_t list_blocks_per_sm;   /* hit-list kernels (temporal, shading requests): blocks per SM (1..64) */
     uint32_t occupancy;            /* 0 or 1; no effect (kernels are built at the register count that measured fastest) */

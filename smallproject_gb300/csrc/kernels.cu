@@ -538,14 +538,17 @@ struct ShadowWarp {
 // walked by the whole warp. Queues are first in, first out, so a ray's earliest hit is the
 // first one seen; its lane takes the answer and any later tasks of it are dropped. A lane
 // is refilled from the request queue once `refill` lanes are done, after both queues
-// have been emptied (an ended walk is a miss only when none of its tasks hit).
+// have been emptied (an ended walk is a miss only when none of its tasks hit): half as many as
+// the tuning says for candidates, a quarter for shading, whose rays are more alike. Passes in
+// us at 8, 4, 3, 2 and 1 idle lanes: 720p candidates 319, 312, 311, 311, 317, shading 304, 291,
+// 288, 285, 279; 1080p 515, 511, 510, 515, 543 and 616, 606, 605, 601, 601.
 // Bound by instruction issue (70 % active at 960 x 540), not by memory (25 MB of DRAM reads):
 // a walker that also steps through bricks keeps 9 of 32 threads busy per instruction, since
 // some lane is always in a brick; with the bricks taken out of the walk and packed densely
 // 18 are, and a ray costs 387 warp instructions instead of 860. 1,894,052 candidate rays of
 // the 1080p frame with 65,536 emitters: 1,563 us before, 728 us now, 515 for the three quarters
-// of them in reach (shading's 1,801,412: 1,330 and 616 us); 58,047 rays of a 333 x 187 frame, bound by the longest ray: 77 and 45
-// us. 7 blocks a SM (72 registers): 6 took 768 us, 8 (64 registers, spills) 755 us.
+// of them in reach (shading's 1,801,412: 1,330 and 601 us); 58,047 rays of a 333 x 187
+// frame, bound by the longest ray: 77 and 45 us. 7 blocks a SM (72 registers): 6 took 768 us, 8 (64 registers, spills) 755 us.
 // BOX: 1 the world has cell boxes and opacity masks, 2 brick boxes only, 0 neither (cells and
 // voxels are read).
 template <int VARIANT, int BOX, int MINB>
@@ -553,6 +556,7 @@ __global__ void __launch_bounds__(128, MINB) shadow_kernel(const __grid_constant
                                                            int planeSel) {
     follow_previous();
     __shared__ ShadowWarp s_warp[4];
+    const int refill = max(bd.refill >> (planeSel ? 2 : 1), 1);
     ShadowWarp& q = s_warp[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
@@ -678,7 +682,7 @@ __global__ void __launch_bounds__(128, MINB) shadow_kernel(const __grid_constant
                         q.cell[slot++ & (kCellQueue - 1u)] = make_uint2(__float_as_uint(ct[u]), cp[u] | ((uint32_t)lane << 23));
             }
             const unsigned busy = __ballot_sync(0xffffffffu, st == GW_UBER || st == GW_GRID);
-            flush = busy == 0u || (!exhausted && 32 - __popc(busy) >= bd.refill);
+            flush = busy == 0u || (!exhausted && 32 - __popc(busy) >= refill);
             __syncwarp();
             while (n1 >= 32u || (flush && n1 > 0u)) {
                 const uint32_t cnt = min(n1, 32u);
