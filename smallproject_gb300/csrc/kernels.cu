@@ -454,8 +454,9 @@ __device__ __forceinline__ float4 path_trace_px(const World& w, const Frame& k, 
     const float NdotL = fmaxf(0.0f, (N.x * R.x + N.y * R.y) + N.z * R.z);
     float dist2 = 0.0f;
     uint32_t side2 = 0;
-    const uint32_t voxel2 = trace_first<1, true, false>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z,
-                                                    128, &dist2, &side2);
+    // (by the bricks' masks: 8 samples at 1080p 9.15 ms -> 8.92; the primary ray by masks too 8.96)
+    const uint32_t voxel2 = trace_first<1, true, true>(w, I.x + 0.1f * N.x, I.y + 0.1f * N.y, I.z + 0.1f * N.z, R.x, R.y, R.z,
+                                                   128, &dist2, &side2);
     const float3 sampleL = mul(mul(to_rgb(voxel2), (float)((voxel2 & 0xff0000u) >> 16)), INVPI);
     const float TWOPI = 6.28318530717958647692528f;
     return make_float4(((sampleL.x * TWOPI) * NdotL) * brdf.x + contribution.x,
