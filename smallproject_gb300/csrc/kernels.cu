@@ -1386,8 +1386,8 @@ __device__ __forceinline__ void shade_finish_px(const ViewDev* V, int x, int y, 
             const float3 sp = f3(D.x * dist + k.E.x, D.y * dist + k.E.y, D.z * dist + k.E.z);
             float dist2 = 0.0f;
             uint32_t side2 = 0;
-            const uint32_t voxel2 = trace<1>(V->w, sp.x + 0.1f * N.x, sp.y + 0.1f * N.y, sp.z + 0.1f * N.z, R.x, R.y, R.z,
-                                             10 /* GRIDWIDTH / 12 */, 0u, 0u, &dist2, &side2);
+            const uint32_t voxel2 = trace_first<1, true, true, true>(V->w, sp.x + 0.1f * N.x, sp.y + 0.1f * N.y, sp.z + 0.1f * N.z,
+                                                                     R.x, R.y, R.z, 10 /* GRIDWIDTH / 12 */, &dist2, &side2);
             float3 toAdd = f3(sky->lightScale, sky->lightScale, sky->lightScale), M = N;
             if (voxel2 != 0u) {
                 const float3 c2 = to_rgb(voxel2);
@@ -1405,8 +1405,11 @@ __device__ __forceinline__ void shade_finish_px(const ViewDev* V, int x, int y, 
     if (fuse) accumulate_px(V, i, px);
 }
 
+// SKY: bound by the 10-step ray's chain of loads, which more warps hide: 1080p 297 us with
+// trace<1> (64 registers), by masks 240 with 80 registers, 204 with 48 (the frame 3.25, 3.17
+// and 3.14 ms). A batch's table variant spills more and keeps 80.
 template <int VARIANT, bool SKY>
-__global__ void __launch_bounds__(kMaxTileThreads) shade_finish_kernel(const __grid_constant__ BatchDev bd) {
+__global__ void __launch_bounds__(kMaxTileThreads, SKY ? (VARIANT < 2 ? 5 : 3) : 1) shade_finish_kernel(const __grid_constant__ BatchDev bd) {
     follow_previous();
     uint32_t tile, round = 0;
     while (next_tile(bd, bd.counters + kCtrFinish, &tile, round)) {

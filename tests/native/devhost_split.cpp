@@ -91,6 +91,18 @@ uint32_t dh_trace_first(const uint32_t* grid, const uint8_t* uber, const uint32_
     return f(w, O[0], O[1], O[2], D[0], D[1], D[2], steps, dist, side);
 }
 
+// trace<1> over cell masks
+uint32_t dh_trace_opaque(const uint32_t* grid, const uint8_t* uber, const uint32_t* bricks, const uint32_t* ucell, const uint32_t* gbox,
+                         const uint32_t* bmask, const float* O, const float* D, int steps, float* dist, uint32_t* side) {
+    World w = make_world(grid, uber, bricks);
+    w.ucell = reinterpret_cast<const unsigned long long*>(ucell);
+    w.gbox = reinterpret_cast<const uint2*>(gbox);
+    w.bmask = bmask;
+    *dist = 0.0f;
+    *side = 0;
+    return trace_first<1, true, true, true>(w, O[0], O[1], O[2], D[0], D[1], D[2], steps, dist, side);
+}
+
 // An area-light candidate: one call (area_candidate) and the two functions it stands for.
 // in: light centre, size, emission rgb, shading point, offset point, normal sign, albedo/pi rgb;
 // out[which]: ph, seed bits, point xyz, weight, face bits. Returns area_candidate's answer.

@@ -224,6 +224,40 @@ def test_trace_first_matches_trace(dh, split, world0_arrays):  # noqa: F811
     assert _compare_first(dh, split, wa, O, D, steps) > 1500
 
 
+def _compare_opaque(dh, split, wa, O, D, stepss):  # noqa: F811
+    P = lambda a: a.ctypes.data  # noqa: E731
+    split.dh_trace_opaque.restype = C.c_uint32
+    split.dh_trace_opaque.argtypes = [C.c_void_p] * 6 + [C.POINTER(C.c_float)] * 2 + [C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_uint32)]
+    boxes, masks = brick_boxes(wa.bricks), brick_masks(wa.bricks)
+    uc = uber_cells(wa.grid, wa.bricks, boxes)
+    gb = np.stack([wa.grid, np.where(wa.grid & 1, boxes[np.where(wa.grid & 1, wa.grid >> 1, 0)], 0).astype(np.uint32)], 1)
+    hits = 0
+    for i in range(len(O)):
+        o, d, steps = _f3(O[i]), _f3(D[i]), int(stepss[i])
+        da, sa, db, sb = C.c_float(0), C.c_uint32(0), C.c_float(0), C.c_uint32(0)
+        a = dh.dh_trace(1, P(wa.grid), P(wa.uber), P(wa.bricks), o, d, steps, 0, 0, C.byref(da), C.byref(sa))
+        b = split.dh_trace_opaque(P(wa.grid), P(wa.uber), P(wa.bricks), P(uc), P(gb), P(masks), o, d, steps, C.byref(db), C.byref(sb))
+        assert a == b, (i, O[i], D[i], steps)
+        if a:
+            assert sa.value == sb.value and np.float32(da.value).view(np.uint32) == np.float32(db.value).view(np.uint32), (i, O[i])
+        hits += a != 0
+    return hits
+
+
+def test_opaque_trace_over_masks_matches_trace(dh, split, world0_arrays):  # noqa: F811
+    """The sky light's ray: terrain, from inside and outside the map and leaving the surface, with
+    its budget of 10, smaller and larger ones; numbers that are not finite."""
+    wa = world0_arrays
+    o1, d1, rng = _rays(1500, 95)
+    o2, d2, _ = _surface_rays(wa, 2500, 96)
+    n, i = np.nan, np.inf
+    d3 = np.float32([[0, -1, 0], [n, n, n], [i, 0, 0], [n, 0, -1], [0.6, n, 0.8], [0, 0, 0]])
+    o3 = np.tile(np.float32([[128.5, 200.5, 128.5]]), (len(d3), 1))
+    O, D = np.concatenate([o1, o2, o3]), np.concatenate([d1, d2, d3])
+    steps = rng.choice([10, 10, 128, 9, 5, 4, 1], len(O))
+    assert _compare_opaque(dh, split, wa, O, D, steps) > 300
+
+
 def test_trace_first_matches_trace_on_solid_cells(dh, split):  # noqa: F811
     """Brick-less cells, bricks without a non-zero voxel, single voxels in the air."""
     import smallproject_gb300 as vx
