@@ -71,11 +71,11 @@ static int upload(World& w) {
     if (!w.dev) w.dev = new DeviceWorld();
     DeviceWorld& d = *w.dev;
     d.device = dev;
-    if (!d.grid) CU(cudaMalloc(&d.grid, kGridSize * sizeof(uint32_t)), "cudaMalloc(grid)");
-    if (!d.uber) CU(cudaMalloc(&d.uber, 32 * 32 * 32), "cudaMalloc(uber)");
-    if (!d.ucell0) CU(cudaMalloc(&d.ucell0, 32 * 32 * 32 * sizeof(uint4)), "cudaMalloc(uber boxes)");
-    if (!d.ucell) CU(cudaMalloc(&d.ucell, 32 * 32 * 32 * sizeof(unsigned long long)), "cudaMalloc(uber cells)");
-    if (!d.gbox) CU(cudaMalloc(&d.gbox, 2 * (size_t)kGridSize * sizeof(uint2)), "cudaMalloc(cell boxes)");
+    if (!d.grid) CU(cudaMalloc(&d.grid, kGridBytes), "cudaMalloc(grid)");
+    if (!d.uber) CU(cudaMalloc(&d.uber, kUberCells), "cudaMalloc(uber)");
+    if (!d.ucell0) CU(cudaMalloc(&d.ucell0, kUberCells * sizeof(uint4)), "cudaMalloc(uber boxes)");
+    if (!d.ucell) CU(cudaMalloc(&d.ucell, kUberCells * sizeof(unsigned long long)), "cudaMalloc(uber cells)");
+    if (!d.gbox) CU(cudaMalloc(&d.gbox, kGridBoxBytes), "cudaMalloc(cell boxes)");
     d.gbox0 = d.gbox + kGridSize;
     uint32_t sent = 0;
     if (full) {
@@ -89,9 +89,9 @@ static int upload(World& w) {
             d.bbox = nullptr;
             d.bmask = nullptr;
             d.cap = 0;
-            CU(cudaMalloc(&d.bricks, (size_t)cap * kBrick * sizeof(uint32_t)), "cudaMalloc(bricks)");
-            CU(cudaMalloc(&d.bbox, (size_t)cap * 2u * sizeof(uint32_t)), "cudaMalloc(brick boxes)");
-            CU(cudaMalloc(&d.bmask, (size_t)cap * 32u * sizeof(uint32_t)), "cudaMalloc(brick masks)");
+            CU(cudaMalloc(&d.bricks, cap * kVoxelBytes), "cudaMalloc(bricks)");
+            CU(cudaMalloc(&d.bbox, cap * kBrickBoxBytes), "cudaMalloc(brick boxes)");
+            CU(cudaMalloc(&d.bmask, cap * kBrickMaskBytes), "cudaMalloc(brick masks)");
             d.cap = cap;
         }
         d.bbox0 = d.bbox + d.cap;
@@ -110,7 +110,7 @@ static int upload(World& w) {
             d.stageDev = nullptr;
             d.stageCap = 0;
             const uint32_t cap = std::max<uint32_t>(w.dirtyCount + w.dirtyCount / 2u, 64u);
-            const size_t bytes = (size_t)cap * (kBrick + 1u) * sizeof(uint32_t);
+            const size_t bytes = cap * kStageBytes;
             CU(cudaMallocHost(&d.stageHost, bytes), "cudaMallocHost(commit staging)");
             CU(cudaMalloc(&d.stageDev, bytes), "cudaMalloc(commit staging)");
             d.stageCap = cap;
@@ -493,9 +493,10 @@ int vxr_world_pending(const vxr_world* w, uint32_t* dirty_bricks, int* grid_chan
 int vxr_world_device_bytes(const vxr_world* w, uint64_t* bytes) {
     VXR_CHECK_ARG(w && bytes, "vxr_world_device_bytes: null argument");
     const vxr::DeviceWorld* d = w->w.dev;
-    // grid and its two box tables, uber grid and its masks, bricks, their boxes and masks, light tables
-    *bytes = d ? (uint64_t)(vxr::kGridSize * 20 + 32768 + 32768 * 16 + 32768 * 8 + (uint64_t)d->cap * (vxr::kBrick * 4 + 8 + 64) +
-                            (uint64_t)d->stageCap * (vxr::kBrick + 1) * 4 + d->lcap * 48)
+    *bytes = d ? vxr::kGridBytes + vxr::kGridBoxBytes +
+                     vxr::kUberCells * (sizeof(uint8_t) + sizeof(uint4) + sizeof(unsigned long long)) +
+                     d->cap * (vxr::kVoxelBytes + vxr::kBrickBoxBytes + vxr::kBrickMaskBytes) +
+                     d->stageCap * vxr::kStageBytes + d->lcap * (sizeof(uint4) + 2 * sizeof(float4))
                : 0;
     return VXR_OK;
 }

@@ -10,6 +10,15 @@
 #include "world.hpp"
 
 namespace vxr {
+// What a world's GPU copy holds, in bytes: the allocations and vxr_world_device_bytes take it
+// from here. Per grid cell its value and the two box tables' entries (gbox, gbox0), per uber
+// cell the occupancy byte and the entries of ucell0 and ucell, per brick of the pool its
+// voxels, its two boxes and its two masks of 16 words, per light its record and the two tables.
+constexpr size_t kUberCells = 32 * 32 * 32;
+constexpr size_t kGridBytes = kGridSize * sizeof(uint32_t), kGridBoxBytes = 2 * (size_t)kGridSize * sizeof(uint2);
+constexpr size_t kVoxelBytes = kBrick * sizeof(uint32_t), kBrickBoxBytes = 2 * sizeof(uint32_t),
+                 kBrickMaskBytes = 2 * 16 * sizeof(uint32_t);
+constexpr size_t kStageBytes = (kBrick + 1) * sizeof(uint32_t);   // per staged brick: its voxels and its index
 // GPU copy of a World (runtime.cu)
 struct DeviceWorld {
     uint32_t* grid = nullptr;
