@@ -294,11 +294,11 @@ void free_view(vxr_view* v) {
     if (v->stream) cudaStreamDestroy(v->stream);
 }
 
-// Accumulate the stage durations of the frames before `upto` (finished ones) still in the ring.
-void harvest(vxr_view* v, uint64_t upto) {
+// Accumulate the stage durations of every finished frame still in the ring.
+void harvest(vxr_view* v) {
     const uint64_t from = v->frameSerial > (uint64_t)vxr_view::kRing ? std::max(v->harvested, v->frameSerial - vxr_view::kRing)
                                                                        : v->harvested;
-    for (uint64_t f = from; f < upto; f++) {
+    for (uint64_t f = from; f < v->frameSerial; f++) {
         const int slot = (int)(f % vxr_view::kRing);
         for (int s = 1; s <= 5; s++) {
             const int i = slot * 6 + s;
@@ -308,21 +308,11 @@ void harvest(vxr_view* v, uint64_t upto) {
                 v->statSum[s] += ms;
                 v->statCount[s]++;
             }
+            v->ringMs[i] = ms;
             v->ringUsed[i] = 0;
         }
     }
-    v->harvested = std::max(v->harvested, upto);
-}
-
-// the stage times of the last waited frame, from its ring entries
-void settle_times(vxr_view* v) {
-    if (!v->timesDue) return;
-    v->timesDue = false;
-    for (int s = 1; s <= 5; s++) {
-        const int ri = v->waitedRan[s];
-        v->times[s - 1] = 0.0f;
-        if (ri >= 0) cudaEventElapsedTime(&v->times[s - 1], v->ringFrom[ri], v->ringE[ri]);
-    }
+    v->harvested = v->frameSerial;
 }
 
 // the view's device error flags, reported once
@@ -573,8 +563,8 @@ int vxr_view_create(vxr_world* w, const vxr_view_desc* d, vxr_view** out) {
     v->ringE.assign(vxr_view::kRing * 6, nullptr);
     v->ringFrom.assign(vxr_view::kRing * 6, nullptr);
     v->ringUsed.assign(vxr_view::kRing * 6, 0);
+    v->ringMs.assign(vxr_view::kRing * 6, 0.0f);
     std::fill(std::begin(v->ran), std::end(v->ran), -1);
-    std::fill(std::begin(v->waitedRan), std::end(v->waitedRan), -1);
     for (int i = 0; i < vxr_view::kRing * 6 && e == cudaSuccess; i++) {
         e = cudaEventCreate(&v->ringS[i]);
         if (e == cudaSuccess) e = cudaEventCreate(&v->ringE[i]);
@@ -705,9 +695,6 @@ int vxr_view_begin_frame(vxr_view* v, vxr_frame_consts* out) {
     std::swap(v->buf.qB, v->buf.qBAlt);
     std::swap(v->buf.counters, v->buf.countersAlt);
     if (int r = vxr::brick_cache_begin(v)) return r;
-    // the ring slot this frame takes may hold a waited frame whose times are not worked out yet
-    if (v->frameSerial + 1 - v->waitedSerial >= (uint64_t)vxr_view::kRing) vxr::settle_times(v);
-    if (v->frameSerial - v->harvested >= (uint64_t)vxr_view::kRing && v->harvested < v->waitedSerial) harvest(v, v->waitedSerial);
     v->frameOpen = true;
     std::fill(std::begin(v->ran), std::end(v->ran), -1);
     if (out) *out = k;
@@ -831,10 +818,14 @@ int vxr_view_render(vxr_view* v) {
 static int view_wait(vxr_view* v, bool join) {
     if (join) vxr::proposal_join(v);
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_wait");
-    // (stage times are worked out when they are asked for, or when the ring comes round)
-    std::copy(std::begin(v->ran), std::end(v->ran), v->waitedRan);
-    v->timesDue = true;
-    v->waitedSerial = v->frameSerial;
+    harvest(v);   // four event queries a frame, below 0.1 us each
+    for (int s = 1; s <= 5; s++) {
+        const int i = v->ran[s];
+        float ms = i >= 0 ? v->ringMs[i] : 0.0f;
+        // (a frame still open is harvested once it has ended)
+        if (i >= 0 && v->ringUsed[i] && cudaEventElapsedTime(&ms, v->ringFrom[i], v->ringE[i]) != cudaSuccess) ms = 0.0f;
+        v->times[s - 1] = ms;
+    }
     // kernel times once every marked kernel has run (the training step's marks are on its
     // side stream)
     if (v->ktimer && join) v->ktimer->harvest();
@@ -849,7 +840,6 @@ int vxr_view_wait(vxr_view* v) {
 int vxr_view_stage_times(vxr_view* v, float ms[5]) {
     if (int r = check_view(v, "vxr_view_stage_times")) return r;
     VXR_CHECK_ARG(ms, "vxr_view_stage_times: null output");
-    vxr::settle_times(v);
     for (int i = 0; i < 5; i++) ms[i] = v->times[i];
     return VXR_OK;
 }
@@ -1231,8 +1221,7 @@ extern "C" int vxr_view_stage_stats(vxr_view* v, double sum_ms[5], uint32_t coun
     if (int r = check_view(v, "vxr_view_stage_stats")) return r;
     VXR_CHECK_ARG(sum_ms && count, "vxr_view_stage_stats: null output");
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_stage_stats");
-    v->waitedSerial = v->frameSerial;
-    harvest(v, v->frameSerial);
+    harvest(v);
     for (int s = 1; s <= 5; s++) {
         sum_ms[s - 1] = v->statSum[s];
         count[s - 1] = v->statCount[s];

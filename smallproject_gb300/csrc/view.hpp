@@ -104,7 +104,8 @@ struct vxr_view {
     static constexpr int kRing = 256;
     std::vector<cudaEvent_t> ringS, ringE;             // kRing * 6
     std::vector<cudaEvent_t> ringFrom;                 // kRing * 6: the event a stage's time starts at
-    std::vector<uint8_t> ringUsed;                     // kRing * 6
+    std::vector<uint8_t> ringUsed;                     // kRing * 6: recorded, not harvested yet
+    std::vector<float> ringMs;                         // kRing * 6: what the harvest found
     uint64_t frameSerial = 0, harvested = 0;
     double statSum[6] = {};
     uint32_t statCount[6] = {};
@@ -126,10 +127,7 @@ struct vxr_view {
     bool frameOpen = false;
     vxr_frame_consts k{};
     uint64_t seenLightVersion = 0, seenLightMoveVersion = 0;
-    int waitedRan[6] = {};                            // `ran` of the last waited frame,
-    float times[5] = {};                              // its stage times,
-    bool timesDue = false;                            // still to be worked out
-    uint64_t waitedSerial = 0;                        // frames before it have been waited for
+    float times[5] = {};                              // stage times of the last waited frame
     // device error flags, in page-locked memory the kernels write through buf.err: reading them
     // after a wait is a load
     volatile uint32_t* errHost = nullptr;
@@ -143,7 +141,7 @@ dev::World dev_world(vxr_view* v);
 dev::Frame dev_frame(const vxr_frame_consts& c);
 int ensure_world(vxr_view* v);
 void free_view(vxr_view* v);
-void harvest(vxr_view* v, uint64_t upto);
+void harvest(vxr_view* v);
 int report_flags(vxr_view* v);
 Tuning shape(const vxr_view* v);
 int check_tuning(const vxr_tuning* t, const char* fn);
