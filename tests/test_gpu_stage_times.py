@@ -17,15 +17,15 @@ def _frame(v, f):
 
 def test_stage_times_stay_those_of_the_waited_frame(lib, cuda_device, scene0):
     w, _ = scene0
-    v = lib.View(w, lib.view_desc(320, 180, lib.LIGHTS_AREA, num_candidates=1024))
+    v = lib.View(w, lib.view_desc(1280, 720, lib.LIGHTS_AREA, num_candidates=64))
     try:
         for f in range(3):
             _frame(v, f)
             v.wait()
-        long = v.stage_times()[1]                 # 1,024 candidates
+        long = v.stage_times()[1]                 # 64 candidates (the scene's emitters)
         _frame(v, 3)
         v.wait()                                  # the last waited frame
-        v.set_params(lib.view_desc(320, 180, lib.LIGHTS_AREA, num_candidates=1))
+        v.set_params(lib.view_desc(1280, 720, lib.LIGHTS_AREA, num_candidates=1))
         for f in range(200):
             _frame(v, f)
         v.stage_stats()                           # waits for the view, and is no vxr_view_wait
