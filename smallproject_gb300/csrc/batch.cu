@@ -350,10 +350,7 @@ int vxr_batch_wait(vxr_batch* b, float* ms) {
         if (b->timed && cudaEventElapsedTime(ms, b->t0, b->t1) != cudaSuccess) *ms = 0.0f;
     }
     uint32_t any = 0;
-    for (vxr_view* v : b->views) {
-        any |= *v->errHost;
-        *v->errHost = 0u;
-    }
+    for (vxr_view* v : b->views) any |= vxr::take_flags(v, 0xFFFFFFFFu);
     if (any)
         return vxr::set_error(VXR_E_DEVICE, vxr::device_flags_message(any));
     return VXR_OK;

@@ -42,6 +42,7 @@ namespace vxr {
 namespace dev {
 
 __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t code) { atomicOr(err, code); }
+__global__ void clear_flags_kernel(uint32_t* err, uint32_t flags) { atomicAnd(err, ~flags); }
 
 // The start of every kernel that launch_next may launch: waits until the kernel before it in the
 // stream has ended and its writes are seen (nothing, for a kernel launched plainly).
@@ -1581,6 +1582,8 @@ void launch_build_brick_boxes(const uint32_t* bricks, const uint32_t* list, uint
         launch_next(true, dev::build_brick_boxes_kernel, (unsigned)((threads + 255u) / 256u), 256, s, bricks, list, n, bbox, bbox0, bmask,
                     bmask0);
 }
+
+void launch_clear_flags(uint32_t* err, uint32_t flags, cudaStream_t s) { dev::clear_flags_kernel<<<1, 1, 0, s>>>(err, flags); }
 
 void launch_commit_bricks(const uint32_t* list, const uint32_t* voxels, uint32_t n, uint32_t* bricks, cudaStream_t s) {
     if (n) dev::commit_bricks_kernel<<<n, 128, 0, s>>>(list, voxels, bricks);

@@ -132,6 +132,7 @@ size_t brick_cache_smem(int log2);   // shared memory of the shadow tracer's bri
 void launch_build_light_table(const uint32_t* raw, int words, uint32_t n, float4* geom, float4* emit, cudaStream_t s);
 void launch_build_brick_boxes(const uint32_t* bricks, const uint32_t* list, uint32_t n, uint32_t* bbox, uint32_t* bbox0,
                               uint32_t* bmask, uint32_t* bmask0, cudaStream_t s);
+void launch_clear_flags(uint32_t* err, uint32_t flags, cudaStream_t s);
 void launch_commit_bricks(const uint32_t* list, const uint32_t* voxels, uint32_t n, uint32_t* bricks, cudaStream_t s);
 // the tables that follow from the grid (kernels.cu); boxes, gbox, gbox0 and err may be null
 void launch_build_cells(const uint32_t* grid, const uint32_t* bbox, const uint32_t* bbox0, uint8_t* uber,

@@ -737,8 +737,7 @@ int vxr_view_proposal_probs(vxr_view* v, uint32_t n, const float* samples, float
     a.err = v->buf.err;
     cudaError_t e = vxr::prop::launch_infer(a, n, v->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(v->stream);
-    if (e == cudaSuccess && (*v->errHost & 16u)) {
-        *v->errHost = 0u;
+    if (e == cudaSuccess && vxr::take_flags(v, 16u)) {
         cudaFree(ds);
         cudaFree(dp);
         return set_error(VXR_E_DEVICE, "vxr_view_proposal_probs: a tensor-core wait gave up");

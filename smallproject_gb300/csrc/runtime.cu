@@ -315,12 +315,21 @@ void harvest(vxr_view* v) {
     v->harvested = v->frameSerial;
 }
 
+// The raised ones among the view's device error flags `which`, cleared. Frames in flight may be
+// raising others: the device clears these alone, after the frames enqueued so far, so that
+// a flag of those frames counts as reported now and one of a later frame stays.
+uint32_t take_flags(vxr_view* v, uint32_t which) {
+    const uint32_t flags = *v->errHost & which;
+    if (!flags) return 0u;
+    launch_clear_flags(v->buf.err, flags, v->stream);
+    cudaStreamSynchronize(v->stream);
+    return flags;
+}
+
 // the view's device error flags, reported once
 int report_flags(vxr_view* v) {
-    const uint32_t err = *v->errHost;
-    if (!err) return VXR_OK;
-    *v->errHost = 0u;
-    return set_error(VXR_E_DEVICE, device_flags_message(err));
+    const uint32_t err = take_flags(v, 0xFFFFFFFFu);
+    return err ? set_error(VXR_E_DEVICE, device_flags_message(err)) : VXR_OK;
 }
 
 void ViewKernelTimer::mark(int k, bool end, cudaStream_t s) {

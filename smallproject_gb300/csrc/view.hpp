@@ -129,7 +129,8 @@ struct vxr_view {
     uint64_t seenLightVersion = 0, seenLightMoveVersion = 0;
     float times[5] = {};                              // stage times of the last waited frame
     // device error flags, in page-locked memory the kernels write through buf.err: reading them
-    // after a wait is a load
+    // after a wait is a load. Only the device writes it (take_flags), as atomics of later
+    // frames may be under way.
     volatile uint32_t* errHost = nullptr;
     size_t npx = 0;
 };
@@ -142,6 +143,7 @@ dev::Frame dev_frame(const vxr_frame_consts& c);
 int ensure_world(vxr_view* v);
 void free_view(vxr_view* v);
 void harvest(vxr_view* v);
+uint32_t take_flags(vxr_view* v, uint32_t which);
 int report_flags(vxr_view* v);
 Tuning shape(const vxr_view* v);
 int check_tuning(const vxr_tuning* t, const char* fn);
