@@ -228,7 +228,8 @@ __device__ __forceinline__ uint32_t append_slot(uint32_t* counter) {
 
 // Block-aggregated append: one atomic per block and call instead of one per warp, so a
 // list filled by a short kernel is not serialised on its counter. Every thread of the
-// block calls it (flag = this thread appends); returns this thread's slot when flag.
+// block, which has whole warps (the ballot waits for all 32 lanes), calls it (flag = this
+// thread appends); returns this thread's slot when flag.
 __device__ __forceinline__ uint32_t block_append(uint32_t* counter, bool flag) {
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_base;

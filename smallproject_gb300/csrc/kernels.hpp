@@ -102,7 +102,7 @@ struct BatchDev {
     int bcLog2 = 0;
     int fuse = 0;                         // shading also accumulates
     int lists = 0;                        // a whole frame, stages 1 to 4 in order: the counters are cleared once, and lists
-                                          // are filled by the kernels that have their entries at hand
+                                          // are filled by the kernels that have their entries at hand (tiles of whole warps only)
     int grouped = 0;                      // a block's hits are listed by the axis of their face
     int cleared = 0;                      // a whole frame's counters are zero already
     int sky = 0;                          // some view has a sky dome (shading runs its variant)

@@ -722,8 +722,8 @@ int vxr_view_set_frame_consts(vxr_view* v, const vxr_frame_consts* k) {
 }
 
 // fuse: a whole frame's stage (shading accumulates; lists filled by the kernels before them,
-// unless kernels are timed one by one). s: the stream of the stage's launches; tail (candidate stage): the stream of its
-// temporal pass, handed on by an event (null: s)
+// unless kernels are timed one by one). s: the stream of the stage's launches; tail
+// (candidate stage): the stream of its temporal pass, handed on by an event (null: s)
 static int run_stage(vxr_view* v, int stage, bool fuse, cudaStream_t s, cudaStream_t tail = nullptr) {
     if (!tail) tail = s;
     if (!v->frameOpen) return set_error(VXR_E_STATE, "vxr_view_stage: call vxr_view_begin_frame first");
@@ -750,7 +750,9 @@ static int run_stage(vxr_view* v, int stage, bool fuse, cudaStream_t s, cudaStre
     vxr::BatchDev bd = vxr::single_batch(w, k, v->buf, v->cur, point, sh);
     bd.fuse = fuse ? 1 : 0;
     bd.timer = v->ktimerOn ? v->ktimer : nullptr;
-    bd.lists = fuse && !bd.timer ? 1 : 0;
+    // (lists are appended to by whole blocks, with ballots of whole warps: tiles that leave a
+    // warp broken take the separate list kernels)
+    bd.lists = fuse && !bd.timer && sh.bx * sh.by % 32 == 0 ? 1 : 0;
     if (v->useProposal) bd.grouped = 0;   // its candidates are not scanned
     if (sh.brickCache > 0) {
         if (v->bc.calibrating) {
