@@ -23,7 +23,7 @@ SPACE = [
     ("tile", [(16, 8), (32, 4), (8, 16), (32, 8), (16, 16), (64, 2)]),
     ("persistent", [0, 1]),
     ("shadow_refill", [4, 8, 16, 24]),
-    ("shadow_burst", [2, 4, 8, 16]),
+    ("shadow_burst", [4, 8, 16]),     # the tracer takes bursts in steps of 4 visits
     ("list_blocks_per_sm", [4, 8, 16, 32]),
 ]
 # What vxr_tuning has besides is not searched: occupancy changes nothing, and shadow_schedule,
