@@ -30,8 +30,10 @@ SPACE = [
 # shadow_early_out and brick_cache select the resumable walker, which takes twice as long as
 # the split tracer (1,563 us against 728 for 1.9 million rays at 1080p).
 
-
-KERNELS = "split"
+# Raised with every change of the kernels, or of what a searched value means to them, that
+# makes cached winners stale. (split2: refill counts halved for candidates and quartered
+# for shading, bursts in steps of 4.)
+KERNELS = "split2"
 
 
 def default_cache_path():
