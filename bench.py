@@ -48,7 +48,7 @@ import time
 import numpy as np
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
-# clock samples and the autotuner's cache (VXR_BENCH_OUT overrides the folder)
+# clock samples, the autotuner's cache and the details of a run (VXR_BENCH_OUT overrides the folder)
 OUT_DIR = os.environ.get("VXR_BENCH_OUT", os.path.join(ROOT, "_build"))
 sys.path.insert(0, ROOT)
 
@@ -299,6 +299,32 @@ NFR = 300
 # (profiles/), scaled by 4 to 1920x1080 (the ray count grows with the pixel count)
 NCU_TRAFFIC_1080P = {"shadow_candidates": 4 * (20.84e6 + 0.00e6), "shadow_shading": 4 * (23.44e6 + 0.00e6),
                      "ris_candidates": 4 * (10.37e6 + 0.06e6), "albedo": 4 * (14.66e6 + 2.41e6)}
+
+
+# The one JSON line of a run holds these keys, and of those in LINE_EXTRAS as many, in this order,
+# as fit LINE_MAX bytes: readers keep the end of a program's output, and a line that is
+# longer than that end is lost whole. Everything goes to DETAILS in the output folder.
+LINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+             "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks")
+LINE_EXTRAS = ("plain_ms_per_frame", "cpu_baseline", "roofline", "rays_per_s", "chains", "host_ms_per_frame",
+               "individual_views_host_ms_per_frame")
+LINE_MAX = 2000
+DETAILS = "bench_details.json"
+
+
+def emit(line):
+    """Prints the run's JSON line and writes all of `line` to DETAILS."""
+    os.makedirs(OUT_DIR, exist_ok=True)
+    with open(os.path.join(OUT_DIR, DETAILS), "w") as fh:
+        json.dump(line, fh, indent=1)
+    short = {k: line[k] for k in LINE_KEYS if k in line}
+    for k in LINE_EXTRAS:
+        v = line.get(k)
+        if isinstance(v, dict):
+            v = {a: b for a, b in v.items() if a != "note"}
+        if v is not None and len(json.dumps({**short, k: v})) <= LINE_MAX:
+            short[k] = v
+    print(json.dumps(short))
 
 
 def boot_ci(groups, stat, n=2000, seed=0):
@@ -691,7 +717,7 @@ def run_batch(args, dist, rank, ws, warmup):
             "tuning": rep["tuning"], "tuning_search": rep}
     if learned4 is not None:
         line["learned"] = learned4
-    print(json.dumps(line))
+    emit(line)
     if batch is not None:
         batch.close()
     for v in views:
@@ -1017,7 +1043,7 @@ def main():
             "gpu_launches": launches, "clocks": clk,
             "tuning": view.get_tuning().as_dict(), "tuning_search": tuning_report,
             "modes": modes, "configs_0_1": configs01, "world_commit": world_commit_times(world, args)}
-    print(json.dumps(line))
+    emit(line)
     view.close()
 
 
