@@ -1755,11 +1755,16 @@ void launch_batch_candidates(const BatchDev& bd, int variant, const LearnedHook*
 }
 
 // A whole frame's shading requests come from the spatial pass while the frame is small: that
-// saves a launch and a pass (333 x 187: 265 -> 260 us a frame, 640 x 360: 372 -> 366). From a
-// million pixels on the separate kernel costs less, as it runs beside the next frame's
-// primary rays and the spatial pass keeps its registers (1280 x 720: 15 us a frame less, 1080p
-// 15 us). The line lies between the sizes measured.
-constexpr uint32_t kSpatialRequests = 1u << 19;
+// saves a launch and a pass. In larger frames the pass, with the registers and barriers that
+// appending costs it, holds back the next frame's primary rays, which start at its end and
+// run beside the separate kernel. Frames in us with the pass appending and with the kernel:
+// one after the other 480 x 270 169 and 172 (4,096 emitters 302 and 304), 640 x 360 230 and 232
+// (423 and 427), 720 x 405 261 and 256 (494 and 472), 800 x 450 299 and 293 (577 and 555),
+// 960 x 540 384 and 378 (759 and 743), 1280 x 720 614 and 612 (1,237 and 1,231); each waited
+// for, the pass stays ahead: 640 x 360 268 and 271, 720 x 405 298 and 303 (533 and 537),
+// 960 x 540 426 and 431 (803 and 807). Batches, whose frames do not overlap, are within 1 %
+// either way.
+constexpr uint32_t kSpatialRequests = 1u << 18;
 static bool requests_with_spatial(const BatchDev& bd) { return bd.lists && bd.totalPixels <= kSpatialRequests; }
 
 template <bool LISTS>
