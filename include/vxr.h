@@ -380,7 +380,11 @@ int vxr_view_timer_end(vxr_view* v, float* ms);
  * vxr_kernel_name): albedo, compact_hits, proposal_infer, ris_candidates,
  * shadow_candidates, temporal, spatial, shade_request, shadow_shading, shade_finish,
  * accumulate, proposal_train (a frame's online training steps, gather to Adam, as one
- * timed unit). Stats: summed milliseconds and launch counts since the last reset. */
+ * timed unit). Stats: summed milliseconds and launch counts since the last reset.
+ * While it is on, whole frames list their hits and shading rays by kernels of their own
+ * (compact_hits, shade_request), and each kernel is made ready only when the one before it
+ * has ended: the same results, but not the launches of an untimed frame, and some
+ * microseconds a frame more (times without it: vxr_view_stage_times). */
 #define VXR_KERNEL_COUNT 12
 int vxr_view_kernel_timing(vxr_view* v, int on);
 int vxr_view_kernel_stats(vxr_view* v, double sum_ms[VXR_KERNEL_COUNT], uint32_t count[VXR_KERNEL_COUNT], int reset);
@@ -393,7 +397,8 @@ int vxr_view_work_counts(vxr_view* v, uint32_t counts[3]);
 int vxr_view_render_to_host(vxr_view* v, const float pos[3], const float target[3], float* host_rgba);
 /* The same, pipelined: enqueues the frame and the image copy and returns at once with
  * *ticket; vxr_view_image_wait(v, ticket) returns once that image is in host_rgba (and
- * reports device error flags like vxr_view_wait). Up to 4 images may be in flight (a
+ * reports device error flags like vxr_view_wait: for all frames enqueued by then, which it
+ * then waits for; a flag of a later frame is reported anew). Up to 4 images may be in flight (a
  * fifth call first waits for the oldest); give each in-flight image its own host buffer
  * (page-locked, vxr_host_alloc, for the copy to overlap). Rendering frame f + 1 while the
  * host reads image f hides the host's per-frame work behind the device's. */

@@ -891,6 +891,9 @@ __global__ void __launch_bounds__(CACHE ? 512 : 128, CACHE ? 1 : MINB) shadow_wa
 // one after the other, so that a warp takes as many rounds as its lane with the most of them.
 // A scanned candidate costs a sixth of a worked-out one, so a warp scans on only when a third
 // of its lanes' first two candidates lie behind. SCAN: views that scan (kReachEmitters).
+// 1080p frames scanning and not, us, with 8, 12, 16 and 32 candidates: 1,048,576 emitters 1,724
+// and 1,742, 1,852 and 1,896, 1,973 and 2,042, 2,419 and 2,584; 65,536 emitters 2,061 and
+// 2,053, 2,200 and 2,194, 2,326 and 2,322, 2,795 and 2,797: from 16 on it gains more than it costs.
 constexpr uint32_t kScanMin = 16, kScanMax = 32;   // candidates of a pixel (more: no room)
 struct FrontScan {
     uint32_t jump[128];               // xs_jump(14)
@@ -1538,7 +1541,13 @@ void apply_tuning(BatchDev& bd, const Tuning& tu) {
 // us without and with the test: 65,536 emitters at 1080p 914 + 728 and 1,001 + 521, learned
 // 166 + 738 and 253 + 415; 1,048,576 at 4K 3,568 + 2,330 and 3,892 + 1,108. Worlds with fewer
 // lose: 4,096 emitters at 720p 417 + 320 and 460 + 280, 1,024 in a 512^3 world 411 + 266 and
-// 435 + 266. Single views only: a batch's views share a launch.
+// 435 + 266. Whole 720p frames with the test and without, us: 1024-voxel worlds of 8,192
+// emitters 1,277 and 1,281, 16,384 1,277 and 1,293, 32,768 1,291 and 1,319, 65,536 1,320 and
+// 1,363; 256-voxel ones of 16,384 1,189 and 1,179, 32,768 1,233 and 1,237, 65,536 1,189 and
+// 1,223 (the scan's gain). It loses where rays end within their budget: 512-voxel worlds of
+// 32,768 emitters 1,319 and 1,292, of 65,536 1,386 and 1,361, and small frames (333 x 187, 8
+// candidates: 204 and 201) - 1 to 2 %, for which a rule would need the emitters' extent.
+// Single views only: a batch's views share a launch.
 // The area-light candidates of these views are also scanned for those in front of the surface
 // (FrontScan), and their hits listed by the axis of their face: at 4K, where 63 % of the
 // candidates lie behind, 3,902 us -> 3,061 (3,592 with hits in tile order, as neighbouring
@@ -1607,7 +1616,10 @@ void launch_path_trace(const BatchDev& bd, cudaStream_t s) {
 // frames wait for their longest ray, whose brick walk reads a line instead of a sector a row
 // (333 x 187: 42.5 us -> 35.3, 640 x 360: 41.7 -> 36.3, 1280 x 720: 153 -> 144); larger ones are
 // bound by instructions, of which a mask takes more (1080p: 393 -> 405, 3840 x 2160: 2,106 ->
-// 2,176).
+// 2,176). Whole frames with masks and without, us, 4,096 and 65,536 emitters: 960 x 540 759 and
+// 788, 814 and 838; 1120 x 630 969 and 976, 1,040 and 1,045; 1280 x 720 1,231 and 1,237, 1,320
+// and 1,325; 1440 x 810 1,525 and 1,531, 1,637 and 1,639; 1600 x 900 1,851 and 1,855, 1,987 and
+// 1,988; 1080p 2,608 and 2,612, 2,798 and 2,795: alike from a million pixels on.
 constexpr uint32_t kBitsPixels = 1u << 20;
 void launch_batch_albedo(const BatchDev& bd, int variant, cudaStream_t s) {
     const bool bits = variant != 2 && bd.totalPixels <= kBitsPixels && bd.one.w.bmask0;
