@@ -294,11 +294,11 @@ void free_view(vxr_view* v) {
     if (v->stream) cudaStreamDestroy(v->stream);
 }
 
-// Accumulate the stage durations of every finished frame still in the ring.
-void harvest(vxr_view* v) {
+// Accumulate the stage durations of the frames before `upto` (finished ones) still in the ring.
+void harvest(vxr_view* v, uint64_t upto) {
     const uint64_t from = v->frameSerial > (uint64_t)vxr_view::kRing ? std::max(v->harvested, v->frameSerial - vxr_view::kRing)
                                                                        : v->harvested;
-    for (uint64_t f = from; f < v->frameSerial; f++) {
+    for (uint64_t f = from; f < upto; f++) {
         const int slot = (int)(f % vxr_view::kRing);
         for (int s = 1; s <= 5; s++) {
             const int i = slot * 6 + s;
@@ -312,7 +312,16 @@ void harvest(vxr_view* v) {
             v->ringUsed[i] = 0;
         }
     }
-    v->harvested = v->frameSerial;
+    v->harvested = std::max(v->harvested, upto);
+}
+
+// the stage times of the last waited frame, whose entries are still in the ring
+void settle_times(vxr_view* v) {
+    if (!v->timesDue) return;
+    v->timesDue = false;
+    harvest(v, v->timesOf);
+    const float* ms = &v->ringMs[(size_t)((v->timesOf - 1) % vxr_view::kRing) * 6];
+    std::copy(ms + 1, ms + 6, v->times);
 }
 
 // The raised ones among the view's device error flags `which`, cleared. Frames in flight may be
@@ -704,6 +713,15 @@ int vxr_view_begin_frame(vxr_view* v, vxr_frame_consts* out) {
     std::swap(v->buf.qB, v->buf.qBAlt);
     std::swap(v->buf.counters, v->buf.countersAlt);
     if (int r = vxr::brick_cache_begin(v)) return r;
+    // this frame takes the ring entries of the one kRing frames before it
+    if (v->frameSerial >= (uint64_t)vxr_view::kRing) {
+        const uint64_t old = v->frameSerial - vxr_view::kRing;
+        if (v->timesOf == old + 1) vxr::settle_times(v);
+        if (old >= v->harvested && old < v->waited) harvest(v, old + 1);
+    }
+    const size_t entries = (size_t)(v->frameSerial % vxr_view::kRing) * 6;
+    std::fill_n(v->ringMs.begin() + entries, 6, 0.0f);
+    std::fill_n(v->ringUsed.begin() + entries, 6, (uint8_t)0);
     v->frameOpen = true;
     std::fill(std::begin(v->ran), std::end(v->ran), -1);
     if (out) *out = k;
@@ -828,14 +846,19 @@ int vxr_view_render(vxr_view* v) {
 // overlapping the caller's next frame)
 static int view_wait(vxr_view* v, bool join) {
     if (join) vxr::proposal_join(v);
+    harvest(v, v->waited);
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_wait");
-    harvest(v);   // four event queries a frame, below 0.1 us each
-    for (int s = 1; s <= 5; s++) {
-        const int i = v->ran[s];
-        float ms = i >= 0 ? v->ringMs[i] : 0.0f;
-        // (a frame still open is harvested once it has ended)
-        if (i >= 0 && v->ringUsed[i] && cudaEventElapsedTime(&ms, v->ringFrom[i], v->ringE[i]) != cudaSuccess) ms = 0.0f;
-        v->times[s - 1] = ms;
+    v->waited = v->frameSerial;
+    if (v->frameOpen) {   // (harvested once it has ended)
+        v->timesOf = 0;
+        v->timesDue = false;
+        for (int s = 1; s <= 5; s++) {
+            const int i = v->ran[s];
+            if (i < 0 || cudaEventElapsedTime(&v->times[s - 1], v->ringFrom[i], v->ringE[i]) != cudaSuccess) v->times[s - 1] = 0.0f;
+        }
+    } else if (v->timesOf != v->frameSerial) {
+        v->timesOf = v->frameSerial;
+        v->timesDue = true;
     }
     // kernel times once every marked kernel has run (the training step's marks are on its
     // side stream)
@@ -851,6 +874,7 @@ int vxr_view_wait(vxr_view* v) {
 int vxr_view_stage_times(vxr_view* v, float ms[5]) {
     if (int r = check_view(v, "vxr_view_stage_times")) return r;
     VXR_CHECK_ARG(ms, "vxr_view_stage_times: null output");
+    vxr::settle_times(v);
     for (int i = 0; i < 5; i++) ms[i] = v->times[i];
     return VXR_OK;
 }
@@ -1232,7 +1256,8 @@ extern "C" int vxr_view_stage_stats(vxr_view* v, double sum_ms[5], uint32_t coun
     if (int r = check_view(v, "vxr_view_stage_stats")) return r;
     VXR_CHECK_ARG(sum_ms && count, "vxr_view_stage_stats: null output");
     CUV(cudaStreamSynchronize(v->stream), "vxr_view_stage_stats");
-    harvest(v);
+    v->waited = v->frameSerial;
+    harvest(v, v->frameSerial);
     for (int s = 1; s <= 5; s++) {
         sum_ms[s - 1] = v->statSum[s];
         count[s - 1] = v->statCount[s];

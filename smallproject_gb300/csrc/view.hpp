@@ -99,14 +99,18 @@ struct vxr_view {
     bool spatialEvOk = false;
     cudaEvent_t evs = nullptr, eve = nullptr;         // vxr_view_timer_*
     int ran[6] = {};                                  // per stage: its ring entry in the last frame that ran it, -1 none
-    // per-stage event ring over the last kRing frames, harvested by vxr_view_wait; a stage of
-    // a whole frame starts where the one before it ends, with that one's end event
+    // per-stage event ring over the last kRing frames; a stage of a whole frame starts where the
+    // one before it ends, with that one's end event. A wait harvests the frames that were
+    // waited for before it, while the GPU works on what it waits for (the queries of one
+    // frame after the wait: 2 us of a 212 us frame); whoever asks for times, and a frame
+    // that takes a waited frame's entries, harvests what is left.
     static constexpr int kRing = 256;
     std::vector<cudaEvent_t> ringS, ringE;             // kRing * 6
     std::vector<cudaEvent_t> ringFrom;                 // kRing * 6: the event a stage's time starts at
     std::vector<uint8_t> ringUsed;                     // kRing * 6: recorded, not harvested yet
-    std::vector<float> ringMs;                         // kRing * 6: what the harvest found
+    std::vector<float> ringMs;                         // kRing * 6: what the harvest found (0: stage not run)
     uint64_t frameSerial = 0, harvested = 0;
+    uint64_t waited = 0;                               // frames before this one have been waited for
     double statSum[6] = {};
     uint32_t statCount[6] = {};
     // vxr_view_render_to_host_async: one event per outstanding image, ticket % kImages
@@ -127,7 +131,9 @@ struct vxr_view {
     bool frameOpen = false;
     vxr_frame_consts k{};
     uint64_t seenLightVersion = 0, seenLightMoveVersion = 0;
-    float times[5] = {};                              // stage times of the last waited frame
+    float times[5] = {};                              // stage times of frame timesOf - 1, the last waited one,
+    uint64_t timesOf = 0;                             // (0: of a frame still open)
+    bool timesDue = false;                            // still to be taken from the ring
     // device error flags, in page-locked memory the kernels write through buf.err: reading them
     // after a wait is a load. Only the device writes it (take_flags), as atomics of later
     // frames may be under way.
@@ -142,7 +148,7 @@ dev::World dev_world(vxr_view* v);
 dev::Frame dev_frame(const vxr_frame_consts& c);
 int ensure_world(vxr_view* v);
 void free_view(vxr_view* v);
-void harvest(vxr_view* v);
+void harvest(vxr_view* v, uint64_t upto);
 uint32_t take_flags(vxr_view* v, uint32_t which);
 int report_flags(vxr_view* v);
 Tuning shape(const vxr_view* v);

@@ -79,3 +79,27 @@ def test_no_frame_pays_for_the_times_of_others(lib, cuda_device, scene0):
         assert t[RING::RING].min() <= 2.0 * np.median(t)
     finally:
         v.close()
+
+
+def test_stage_stats_keep_the_last_frames_between_waits(lib, cuda_device, scene0):
+    """300 frames, a wait, 300 frames: of either the last 256 count, whoever harvests them; frames
+    that end otherwise (begun and dropped, without stages) leave nothing behind."""
+    w, _ = scene0
+    v = lib.View(w, lib.view_desc(64, 48, lib.LIGHTS_AREA))
+    try:
+        for f in range(300):
+            _frame(v, f)
+        v.wait()
+        for f in range(300):
+            _frame(v, f)
+        _, counts = v.stage_stats(reset=True)
+        assert list(counts) == [2 * RING] * 4 + [0]
+        v.begin_frame()
+        v.stage(lib.STAGE_ALBEDO)
+        v.begin_frame()                           # the frame before is dropped
+        v.end_frame()
+        v.wait()
+        assert not any(v.stage_times())
+        assert not any(v.stage_stats()[1])
+    finally:
+        v.close()
